@@ -831,7 +831,7 @@ def profile_queues() -> None:
 
 def profile_denoise() -> None:
     """Two recorded frames of the headline scene at 1920x1080, then three
-    bilateral-filter calls (for ncu captures of k_dn_ttest and k_dn_filter)."""
+    bilateral-filter calls (for ncu captures of k_dn_bilateral)."""
     import torch
     dev = torch.device("cuda", 0)
     stream = torch.cuda.Stream(device=dev)
