@@ -99,6 +99,9 @@ private:
 };
 
 constexpr int64_t kMaxPool = int64_t(1) << 21;  // paths in flight
+// Paths left at which k_tail takes over from the wavefront: one path per lane
+// of its resident blocks.
+int tail_limit(int sm_count) { return ar::kTailBlocks * sm_count * ar::kTraceBlock; }
 
 }  // namespace
 
@@ -328,9 +331,6 @@ ar_status run_render(ar_scene* s, const ar_camera* cam, const ar_render_params* 
     ensure_workspace(s, pool, npix);
     PathBuffers B = s->bufs;
     B.capacity = static_cast<int32_t>(pool);
-    ck(cudaMemsetAsync(s->accum, 0, sizeof(double) * 3 * npix, st), "memset accum");
-    ck(cudaMemsetAsync(s->stats, 0, 64, st), "memset stats");
-    ck(cudaMemsetAsync(s->err, 0, 64, st), "memset err");
     if (!s->ev0) { ck(cudaEventCreate(&s->ev0), "event"); ck(cudaEventCreate(&s->ev1), "event"); }
     ck(cudaEventRecord(s->ev0, st), "event record");
     // curand_init of every pixel (a skip-ahead per pixel) only when the stored
@@ -341,44 +341,61 @@ ar_status run_render(ar_scene* s, const ar_camera* cam, const ar_render_params* 
           s->rng_next_frame == fp.frame0))
         ck(launch_rng_init(fp, s->base0, s->base1, s->jump_table67, st), "rng init");
     s->rng_valid = false;
-    ck(launch_pool_init(s->ctl, total, st), "pool init");
+    ck(launch_render_init(s->ctl, total, s->accum, npix, s->stats, s->err, s->sm_count, st), "render init");
     int64_t launches = 2;
     const int grid_trace = s->grid_trace;
     const int grid_other = s->sm_count * 4;
+    const int tail = tail_limit(s->sm_count);
     LaunchTimers tm;
     LaunchTimers* tmp = stats ? &tm : nullptr;
     constexpr int kBatch = 16;
-    // every iteration retires or advances each path by one segment and admits up
-    // to min(pool, npix) new samples (k_plan): a hard bound
-    const int64_t admit = std::max<int64_t>(1, std::min<int64_t>(pool, npix));
-    const int64_t max_iter = (total / admit + 2) * (static_cast<int64_t>(p->max_depth) + 2) + kBatch;
     int cur = 0;
     int64_t iters = 0;
-    int64_t retired = 0;
-    for (;;) {
-        if (tmp) {
-            const size_t need = static_cast<size_t>(2 * (iters + kBatch));
-            for (auto* v : {&s->timer_ext, &s->timer_sh}) {
-                while (v->size() < need) {
-                    cudaEvent_t e;
-                    ck(cudaEventCreate(&e), "event create");
-                    v->push_back(e);
-                }
-            }
-            // the vectors may have grown: re-point; recorded pairs keep their handles
-            tm.extend_ev = s->timer_ext.data();
-            tm.shadow_ev = s->timer_sh.data();
-            tm.cap = static_cast<int>(need / 2);
-        }
-        ck(launch_iterations(s->view, fp, B, s->ctl, s->base0, s->base1, s->jump_table, s->stats, s->ovf, s->err,
-                             s->accum, rec_dev,
-                             kBatch, &cur, grid_trace, grid_other, st, &launches, tmp),
+    if (total <= tail && pool == total) {
+        // few paths, all in one wave: they start at once and k_tail runs them to their
+        // end, with nothing to wait for in between
+        ck(launch_generate(fp, B, s->ctl, s->base0, s->base1, s->jump_table, rec_dev, cur, grid_other, st), "render launch");
+        ck(launch_tail(s->view, fp, B, s->ctl, s->stats, s->ovf, s->err, s->accum, rec_dev, cur, tail, s->sm_count, st),
            "render launch");
-        iters += kBatch;
-        ck(cudaMemcpyAsync(&retired, &s->ctl->retired, sizeof(int64_t), cudaMemcpyDeviceToHost, st), "poll");
-        ck(cudaStreamSynchronize(st), "sync");
-        if (retired >= total) break;
-        if (iters > max_iter) return fail(AR_ERR_DEVICE_FAULT, "path pool did not drain");
+        launches += 3;
+    } else {
+        // every iteration retires or advances each path by one segment and tops
+        // the pool up (k_plan): a hard bound
+        const int64_t max_iter = (total / pool + 2) * (static_cast<int64_t>(p->max_depth) + 2) + kBatch;
+        int64_t left = total;   // samples not yet started
+        for (;;) {
+            // iterations until the host looks again: as many as the samples left
+            // need at least, plus a few to bring the last paths under the tail's
+            // limit (a poll costs about one iteration that has nothing to do)
+            const int batch = static_cast<int>(std::min<int64_t>(kBatch, (left + pool - 1) / pool + 2));
+            if (tmp) {
+                const size_t need = static_cast<size_t>(2 * (iters + batch));
+                for (auto* v : {&s->timer_ext, &s->timer_sh}) {
+                    while (v->size() < need) {
+                        cudaEvent_t e;
+                        ck(cudaEventCreate(&e), "event create");
+                        v->push_back(e);
+                    }
+                }
+                // the vectors may have grown: re-point; recorded pairs keep their handles
+                tm.extend_ev = s->timer_ext.data();
+                tm.shadow_ev = s->timer_sh.data();
+                tm.cap = static_cast<int>(need / 2);
+            }
+            ck(launch_iterations(s->view, fp, B, s->ctl, s->base0, s->base1, s->jump_table, s->stats, s->ovf, s->err,
+                                 s->accum, rec_dev, batch, &cur, grid_trace, grid_other, st, &launches, tmp),
+               "render launch");
+            ck(launch_tail(s->view, fp, B, s->ctl, s->stats, s->ovf, s->err, s->accum, rec_dev, cur, tail, s->sm_count, st),
+               "render launch");
+            ++launches;
+            iters += batch;
+            PoolCtl h;
+            ck(cudaMemcpyAsync(&h, s->ctl, sizeof(h), cudaMemcpyDeviceToHost, st), "poll");
+            ck(cudaStreamSynchronize(st), "sync");
+            if (h.retired >= total) break;
+            left = total - h.gen_next;
+            if (iters > max_iter) return fail(AR_ERR_DEVICE_FAULT, "path pool did not drain");
+        }
     }
     // every pixel's state advanced by one frame per sample (k_regen)
     s->rng_valid = true;
@@ -552,6 +569,7 @@ ar_status ar_scene_create_ex(const ar_object_desc* objects, size_t count, const 
             c0.fov_y_deg = 60.0f;
             const ar::FrameParams f0 = make_frame(s, &c0, nullptr);
             ck(ar::set_intersect_eps(f0.eps_tab), "upload INTERSECT_EPS");
+            ck(ar::set_intersect_eps_tail(f0.eps_tab), "upload INTERSECT_EPS");
         }
         s->objects = static_cast<int64_t>(count);
         s->triangles = hs.triangles;
@@ -1035,11 +1053,8 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
         ck(cudaStreamCreateWithFlags(&w.st, cudaStreamNonBlocking), "stream");
         ck(cudaEventCreateWithFlags(&w.done, cudaEventDisableTiming), "event");
         ck(cudaStreamWaitEvent(w.st, R.fork, 0), "fork");
-        ck(cudaMemsetAsync(w.accum, 0, sizeof(double) * 3 * w.npix, w.st), "memset");
-        ck(cudaMemsetAsync(w.stats, 0, 64, w.st), "memset");
-        ck(cudaMemsetAsync(w.err, 0, 64, w.st), "memset");
         ck(ar::launch_rng_init(w.fp, w.base0, w.base1, jb.scene->jump_table67, w.st), "rng init");
-        ck(ar::launch_pool_init(w.ctl, w.total, w.st), "pool init");
+        ck(ar::launch_render_init(w.ctl, w.total, w.accum, w.npix, w.stats, w.err, jb.scene->sm_count, w.st), "render init");
         ck(cudaEventRecord(w.done, w.st), "event record");
         ck(cudaStreamWaitEvent(st, w.done, 0), "join");
     }

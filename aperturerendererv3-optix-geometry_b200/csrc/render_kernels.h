@@ -12,9 +12,11 @@ namespace ar {
 constexpr int kTraceBlock = 128;  // threads per traversal block (4 warps)
 constexpr int kTraceMinBlocks = 8;  // resident blocks per SM the traversal kernels are built for (<= 64 registers)
 constexpr int kShadeBlock = 256;
+constexpr int kTailBlocks = 3;    // resident blocks per SM of the tail kernel
 
 // Upload INTERSECT_EPS(0..8) to the current device.
 cudaError_t set_intersect_eps(const float* tab9);
+cudaError_t set_intersect_eps_tail(const float* tab9);   // the copy of render_tail.cu
 // Blocks of the persistent traversal kernels: occupancy limit x SM count.
 int trace_grid(int sm_count);
 cudaError_t launch_trace_rays(const SceneView& s, const float4* rays, int n, int any, int32_t* obj, float* t,
@@ -31,7 +33,17 @@ struct LaunchTimers {
     int n_shadow = 0;
 };
 
-cudaError_t launch_pool_init(PoolCtl* ctl, int64_t total, cudaStream_t st);
+// Empty pool for `total` samples, zero sums, counters and error words.
+cudaError_t launch_render_init(PoolCtl* ctl, int64_t total, double* accum, int64_t npix, unsigned long long* stats, int* err,
+                               int sm_count, cudaStream_t st);
+// New samples into the free space of pool `cur` (plan -> regen).
+cudaError_t launch_generate(const FrameParams& fp, const PathBuffers& B, PoolCtl* ctl, uint4* b0, uint2* b1,
+                            const uint32_t* jump_table, ar_path_record* rec, int cur, int grid_other, cudaStream_t st);
+// Runs the paths of pool `cur` to their end when all samples have been started
+// and at most `limit` paths are left, else does nothing (render_tail.cu).
+cudaError_t launch_tail(const SceneView& s, const FrameParams& fp, const PathBuffers& B, PoolCtl* ctl,
+                        unsigned long long* stats, uint32_t* ovf, int* err, double* accum, ar_path_record* rec, int cur,
+                        int limit, int sm_count, cudaStream_t st);
 // `iterations` rounds of plan -> regen -> extend -> shade (per material) -> shadow -> retire.
 cudaError_t launch_iterations(const SceneView& s, const FrameParams& fp, const PathBuffers& B, PoolCtl* ctl,
                               uint4* b0, uint2* b1, const uint32_t* jump_table, unsigned long long* stats,

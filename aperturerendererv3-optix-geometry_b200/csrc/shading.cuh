@@ -301,7 +301,7 @@ __device__ __forceinline__ f3 light_tri_normal(const SceneView& s, int l, f3 p, 
     return dot(n, p - lp) < 0.0f ? -n : n;
 }
 
-__device__ float pdf_light_from_hit(const SceneView& s, int obj, f3 sp, f3 lp, f3 ln, bool tri = false)
+static __device__ float pdf_light_from_hit(const SceneView& s, int obj, f3 sp, f3 lp, f3 ln, bool tri = false)
 {
     const ObjInfo oi = s.objects[obj];
     const float sel = s.light_prob[oi.light];
@@ -354,7 +354,7 @@ struct LightSample {
 };
 
 // NEESampleLight (nee.cuh:330-377) with the box and sphere samplers
-__device__ LightSample sample_light(const SceneView& s, f3 sp, Rng& g, bool tri = false)
+static __device__ LightSample sample_light(const SceneView& s, f3 sp, Rng& g, bool tri = false)
 {
     LightSample ls;
     ls.valid = false;

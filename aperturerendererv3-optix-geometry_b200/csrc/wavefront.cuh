@@ -75,7 +75,8 @@ struct PoolCtl {
     int32_t fetch_ext, fetch_shadow, fetch_rays;  // persistent-kernel work counters
     int32_t plan_new;                   // samples started this iteration
     int32_t plan_base;                  // pool index of the first of them
-    int32_t pad[3];
+    int32_t tail_done;                  // blocks of k_tail that have finished
+    int32_t pad[2];
     int64_t gen_next;                   // next sample index to start (g = s * npix + p)
     int64_t plan_first;                 // sample index of the first path started this iteration
     int64_t retired;                    // paths finished so far
