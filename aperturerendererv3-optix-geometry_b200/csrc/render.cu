@@ -50,29 +50,70 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_trace_rays(Sce
 }
 
 // ------------------------------------------------------------------ RNG
-// curand_init(GLOBAL_SEED, pixelIndex, TOTAL_FRAME_INDEX * 2^32) (random.cuh:35-38)
-// Every pixel's state of InitRand: curand_init(seed, s, frame0 * 2^32) with s
-// its reference pixel index.  One thread per 8x4 pixel block, i.e. per run of
-// 32 consecutive s: curand_init for the block's first pixel, then each next
-// pixel's register as A^(2^67) times the previous one (subsequences are 2^67
-// draws apart; the Weyl counter moves by 362437 * 2^67 = 0 mod 2^32), which
-// replaces 31 of every 32 general skip-aheads by a table jump.
-__global__ void k_rng_init(FrameParams fp, uint4* base0, uint2* base1, const uint32_t* __restrict__ jump67)
+// A uniform jump by the whole warp: lane c looks up chunk c (and c + 32), the
+// contributions meet in a warp-wide XOR.
+__device__ __forceinline__ void xorwow_jump_warp(uint32_t v[5], const uint32_t* __restrict__ table)
 {
-    __shared__ uint32_t jt[kJumpWords];
-    for (int k = threadIdx.x; k < kJumpWords; k += blockDim.x) jt[k] = jump67[k];
+    uint32_t r[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int c = static_cast<int>(lane_id()) + 32 * h;
+        if (c < kJumpChunks) {
+            const uint32_t word = h ? v[4] : (c < 8 ? v[0] : c < 16 ? v[1] : c < 24 ? v[2] : v[3]);
+            const uint32_t* row = table + c * 80 + ((word >> (4 * (c & 7))) & 15u);
+#pragma unroll
+            for (int k = 0; k < 5; ++k) r[k] ^= __ldg(row + 16 * k);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 5; ++k) v[k] = __reduce_xor_sync(0xFFFFFFFFu, r[k]);
+}
+
+// Every pixel's state of InitRand (random.cuh:35-38): curand_init(GLOBAL_SEED, s,
+// frame0 * 2^32) with s its reference pixel index.  The seed's state comes from
+// curand_init without a skip; frame0 and s are then jumps of the register (the
+// Weyl counter moves by 362437 * 2^32 or 2^67 = 0 mod 2^32) along their bits.  A
+// warp takes 8 consecutive 8x4 pixel blocks, i.e. 256 consecutive s: the bits
+// they share are jumped by the warp together, then each lane takes one row of 8
+// pixels of one block: its row's and block's jumps, and one jump per pixel.
+// Bound: latency of the chain of jumps for small images, shared-memory lookups
+// (200 per jump, conflict-free) for large ones.  With one thread per block, its
+// curand_init and 31 jumps one after the other, a 160x120 image took 103 us and
+// 1920x1080 260 us; this takes 14 us and
+// 137 us.
+constexpr int kInitBlock = 128;
+constexpr size_t kInitSmem = static_cast<size_t>(kInitLaneTables) * kJumpWords * 4;
+__global__ void __launch_bounds__(kInitBlock) k_rng_init(FrameParams fp, uint4* base0, uint2* base1,
+                                                         const uint32_t* __restrict__ tables)
+{
+    extern __shared__ __align__(16) uint32_t jt[];
+    const uint32_t* frame_t = tables;
+    const uint32_t* lane_t = tables + kInitFrameBits * kJumpWords;
+    const uint32_t* group_t = lane_t + kInitLaneTables * kJumpWords;
+    for (int k = threadIdx.x; k < kInitLaneTables * kJumpWords / 4; k += kInitBlock)
+        reinterpret_cast<uint4*>(jt)[k] = __ldg(reinterpret_cast<const uint4*>(lane_t) + k);
     __syncthreads();
-    const int grid_y = (fp.height + 3) / 4;
-    const int nblk = fp.grid_x * grid_y;
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nblk; b += gridDim.x * blockDim.x) {
+    const int nblk = fp.grid_x * ((fp.height + 3) / 4);
+    const int groups = (nblk + 7) / 8;
+    const int lane = static_cast<int>(lane_id()), row = lane & 3;
+    for (int w = blockIdx.x * (kInitBlock / 32) + (threadIdx.x >> 5); w < groups; w += gridDim.x * (kInitBlock / 32)) {
         curandStateXORWOW_t st;
-        curand_init(fp.seed, 32ull * static_cast<unsigned long long>(b), fp.frame0 << 32, &st);
+        curand_init(fp.seed, 0, 0, &st);
         uint32_t v[5] = {st.v[0], st.v[1], st.v[2], st.v[3], st.v[4]};
-        const int bx = b % fp.grid_x, by = b / fp.grid_x;
-        for (int w = 0; w < 32; ++w) {   // w = tx + 8 ty: ref_pixel_index order within the block
-            if (w > 0) xorwow_jump(v, jt);   // A^(2^67): the next subsequence
-            const int i = 8 * bx + (w & 7), j = 4 * by + (w >> 3);
-            if (i < fp.width && j < fp.height) {
+        for (uint32_t f = static_cast<uint32_t>(fp.frame0); f; f &= f - 1u)
+            xorwow_jump_warp(v, frame_t + (__ffs(f) - 1) * kJumpWords);
+        for (uint32_t b = static_cast<uint32_t>(w); b; b &= b - 1u)
+            xorwow_jump_warp(v, group_t + (__ffs(b) - 1) * kJumpWords);
+#pragma unroll 1
+        for (int k = 0; k < 5; ++k)   // rows 1 and 2 of 4, then blocks 1, 2 and 4 of 8
+            if ((lane >> k) & 1) xorwow_jump(v, jt + (1 + k) * kJumpWords);
+        const int b = 8 * w + (lane >> 2);
+        const int bx = b % fp.grid_x, j = 4 * (b / fp.grid_x) + row;
+#pragma unroll 1
+        for (int x = 0; x < 8; ++x) {
+            if (x) xorwow_jump(v, jt);
+            const int i = 8 * bx + x;
+            if (b < nblk && i < fp.width && j < fp.height) {
                 const int p = j * fp.width + i;
                 base0[p] = make_uint4(st.d, v[0], v[1], v[2]);
                 base1[p] = make_uint2(v[3], v[4]);
@@ -453,10 +494,13 @@ cudaError_t launch_trace_rays(const SceneView& s, const float4* rays, int n, int
     return cudaGetLastError();
 }
 
-cudaError_t launch_rng_init(const FrameParams& fp, uint4* b0, uint2* b1, const uint32_t* jump67, cudaStream_t st)
+cudaError_t launch_rng_init(const FrameParams& fp, uint4* b0, uint2* b1, const uint32_t* tables, int sm_count, cudaStream_t st)
 {
-    const int nblk = fp.grid_x * ((fp.height + 3) / 4);
-    k_rng_init<<<(nblk + 127) / 128, 128, 0, st>>>(fp, b0, b1, jump67);
+    const cudaError_t e = cudaFuncSetAttribute(k_rng_init, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kInitSmem));
+    if (e != cudaSuccess) return e;
+    const int groups = (fp.grid_x * ((fp.height + 3) / 4) + 7) / 8;
+    const int grid = std::min((groups + kInitBlock / 32 - 1) / (kInitBlock / 32), 2 * sm_count);
+    k_rng_init<<<grid, kInitBlock, kInitSmem, st>>>(fp, b0, b1, tables);
     return cudaGetLastError();
 }
 

@@ -51,8 +51,9 @@ inline Bits160 mat_apply(const Mat160& m, const Bits160& v)
     return r;
 }
 
-// Table of A^(2^p) for the device apply (layout [chunk][word][nibble]).
-inline std::vector<uint32_t> xorwow_jump_table_pow2(int p)
+// The tables of A^(2^p) for several ascending p, one after the other, for the
+// device apply (layout [chunk][word][nibble] each).
+inline std::vector<uint32_t> xorwow_jump_tables(const std::vector<int>& exponents)
 {
     Mat160 m;
     for (int i = 0; i < 160; ++i) {
@@ -60,21 +61,44 @@ inline std::vector<uint32_t> xorwow_jump_table_pow2(int p)
         e.w[i >> 5] = 1u << (i & 31);
         m.col[i] = xorwow_register_step(e);
     }
-    for (int sq = 0; sq < p; ++sq) {  // A^(2^(k+1)) = A^(2^k) * A^(2^k)
-        Mat160 n;
-        for (int i = 0; i < 160; ++i) n.col[i] = mat_apply(m, m.col[i]);
-        m = n;
-    }
-    std::vector<uint32_t> t(kJumpWords, 0u);
-    for (int c = 0; c < kJumpChunks; ++c)
-        for (int nib = 0; nib < 16; ++nib) {
-            Bits160 acc = {{0, 0, 0, 0, 0}};
-            for (int b = 0; b < 4; ++b)
-                if ((nib >> b) & 1)
-                    for (int k = 0; k < 5; ++k) acc.w[k] ^= m.col[4 * c + b].w[k];
-            for (int k = 0; k < 5; ++k) t[(c * 5 + k) * 16 + nib] = acc.w[k];
+    std::vector<uint32_t> t(exponents.size() * kJumpWords, 0u);
+    int have = 0;   // m = A^(2^have)
+    for (size_t q = 0; q < exponents.size(); ++q) {
+        for (; have < exponents[q]; ++have) {  // A^(2^(k+1)) = A^(2^k) * A^(2^k)
+            Mat160 n;
+            for (int i = 0; i < 160; ++i) n.col[i] = mat_apply(m, m.col[i]);
+            m = n;
         }
+        uint32_t* out = t.data() + q * kJumpWords;
+        for (int c = 0; c < kJumpChunks; ++c)
+            for (int nib = 0; nib < 16; ++nib) {
+                Bits160 acc = {{0, 0, 0, 0, 0}};
+                for (int b = 0; b < 4; ++b)
+                    if ((nib >> b) & 1)
+                        for (int k = 0; k < 5; ++k) acc.w[k] ^= m.col[4 * c + b].w[k];
+                for (int k = 0; k < 5; ++k) out[(c * 5 + k) * 16 + nib] = acc.w[k];
+            }
+    }
     return t;
+}
+
+// Table of A^(2^p).
+inline std::vector<uint32_t> xorwow_jump_table_pow2(int p) { return xorwow_jump_tables({p}); }
+
+// Jumps of the per-pixel initialisation (k_rng_init), in units of one curand
+// subsequence (2^67 draws): 1 (the next pixel of a row of 8), 8 and 16 (rows of
+// an 8x4 pixel block), 32, 64 and 128 (blocks of a group of 8), then 256 2^k for
+// the bits of the group index (images have at most 2^28 pixels); before them the
+// frame bits, 2^32 2^k draws.
+constexpr int kInitFrameBits = 31, kInitLaneTables = 6, kInitGroupBits = 22;
+constexpr int kInitTables = kInitFrameBits + kInitLaneTables + kInitGroupBits;
+inline std::vector<uint32_t> xorwow_init_tables()
+{
+    std::vector<int> e;
+    for (int k = 0; k < kInitFrameBits; ++k) e.push_back(32 + k);
+    for (int k : {0, 3, 4, 5, 6, 7}) e.push_back(67 + k);
+    for (int k = 0; k < kInitGroupBits; ++k) e.push_back(67 + 8 + k);
+    return xorwow_jump_tables(e);
 }
 
 // Host apply of a table built by xorwow_jump_table_pow2.
