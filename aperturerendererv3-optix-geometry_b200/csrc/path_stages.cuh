@@ -91,6 +91,14 @@ static __device__ __noinline__ float medium_collision(const SceneView& s, const 
     return delta_track(s.medium, o, d, tmax, h);
 }
 
+// Whether a path's closest-hit query is the solo trace of the medium's object
+// (render.cuh:91-94).
+__device__ __forceinline__ bool extend_solo(const SceneView& s, float4 d4, const uint4& rng1)
+{
+    const int mobj = static_cast<int>(rng1.z);
+    return (ibits(d4.w) & kFlagInside) && mobj >= 0 && s.objects[mobj].type != AR_OBJ_TRIANGLE;
+}
+
 // The start of a path's closest-hit query (Trace, render.cuh:86-99): true when
 // the BVH has to be traversed with r, false when the query was the solo trace
 // of the medium's object (render.cuh:91-94, intersection.cuh:185-193), whose
@@ -100,14 +108,12 @@ __device__ __forceinline__ bool extend_begin(const SceneView& s, float4 o4, floa
 {
     const f3 o = xyz(o4), d = xyz(d4);
     const float e = c_eps_tab[min(ibits(o4.w) >> 16, 8)];
-    if (ibits(d4.w) & kFlagInside) {
+    if (extend_solo(s, d4, rng1)) {
         const int mobj = static_cast<int>(rng1.z);
-        if (mobj >= 0 && s.objects[mobj].type != AR_OBJ_TRIANGLE) {
-            const float t = (kExt && s.objects[mobj].type == AR_OBJ_SDF) ? sdf_solo_t(s, mobj, o, d, e)
-                                                                         : isect_analytic_t(s, mobj, o, d);
-            hit = t >= 0.0f && !(t < e) ? make_int4(mobj, -1, ibits(t), 0) : make_int4(-1, -1, 0, 0);
-            return false;
-        }
+        const float t = (kExt && s.objects[mobj].type == AR_OBJ_SDF) ? sdf_solo_t(s, mobj, o, d, e)
+                                                                     : isect_analytic_t(s, mobj, o, d);
+        hit = t >= 0.0f && !(t < e) ? make_int4(mobj, -1, ibits(t), 0) : make_int4(-1, -1, 0, 0);
+        return false;
     }
     ray_begin(r, o, d, e, INFINITY);
     return true;

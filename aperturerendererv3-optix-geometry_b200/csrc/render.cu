@@ -267,6 +267,8 @@ __global__ void k_regen(FrameParams fp, PathBuffers B, PoolCtl* ctl, int cur, ui
 }
 
 // ------------------------------------------------------------------ extend
+// Scenes with SDF objects or a medium (kExt): this kernel leaves the BVH's hit,
+// k_extend_finish does the rest.
 template <bool kExt>
 struct ExtendIO {
     const PathRec* pool;
@@ -274,7 +276,6 @@ struct ExtendIO {
     int32_t* shade_count;
     int32_t* qsh;
     int cap;
-    uint32_t medium_key;  // medium_frame_key of the render
     // queue the path for shading, bucketed by what it hit (render.cuh:97-118)
     __device__ __forceinline__ void to_shade(const SceneView& s, int k, const int4& h)
     {
@@ -283,27 +284,31 @@ struct ExtendIO {
     }
     __device__ __forceinline__ int load(const SceneView& s, int k, RayState& r)
     {
+        if (kExt) {
+            const float4 o4 = pool[k].o, d4 = pool[k].d;
+            if (extend_solo(s, d4, pool[k].rng1)) return -1;
+            ray_begin(r, xyz(o4), xyz(d4), c_eps_tab[min(ibits(o4.w) >> 16, 8)], INFINITY);
+            return k;
+        }
         int4 h;
-        if (extend_begin<kExt>(s, pool[k].o, pool[k].d, pool[k].rng1, r, h)) return k;
+        if (extend_begin<false>(s, pool[k].o, pool[k].d, pool[k].rng1, r, h)) return k;
         to_shade(s, k, h);
         return -1;
     }
     __device__ __forceinline__ void store(const SceneView& s, int k, const RayState& r)
     {
-        to_shade(s, k, extend_end<kExt>(s, pool[k], r, medium_key));
+        if (kExt) hit[k] = make_int4(r.best.obj, r.best.prim, ibits(r.best.t), 0);
+        else to_shade(s, k, extend_end<false>(s, pool[k], r, 0u));
     }
 };
 
-// Trace's closest-hit query (render.cuh:86-99) for every path of the pool,
-// then (extension) free-flight sampling in the participating medium.
+// Trace's closest-hit query (render.cuh:86-99) for every path of the pool.
 template <bool kExt>
 __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_extend(SceneView s, PathBuffers B, int cur, PoolCtl* ctl,
-                                                        unsigned long long* stats, uint32_t* ovf, int* err,
-                                                        uint32_t medium_key)
+                                                        unsigned long long* stats, uint32_t* ovf, int* err)
 {
     extern __shared__ uint32_t smem[];
     ExtendIO<kExt> io;
-    io.medium_key = medium_key;
     io.pool = pool_of(B, cur);
     io.hit = B.hit;
     io.shade_count = ctl->shade_count;
@@ -312,6 +317,32 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_extend(SceneVi
     const int n = ctl->count[cur];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&stats[0], static_cast<unsigned long long>(n));
     traverse_queue<false>(s, io, n, &ctl->fetch_ext, lane_stack(smem), thread_overflow(ovf), err, &stats[2]);
+}
+
+// The rest of Trace in scenes with SDF objects or a medium: solo traces, SDF
+// objects, free-flight sampling, shading buckets.  A kernel of its own because
+// these loops (sphere tracing, delta tracking) are long and run here with all
+// lanes of a warp; at the refill point of the traversal only the 8 or so lanes
+// whose rays had just finished ran them while the others waited (1280x720, 16
+// samples, four wavelengths: EXT_MEASURED).
+__global__ void __launch_bounds__(kTraceBlock) k_extend_finish(SceneView s, PathBuffers B, int cur, PoolCtl* ctl, uint32_t medium_key)
+{
+    const PathRec* pool = pool_of(B, cur);
+    const int n = ctl->count[cur];
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const PathRec pr = pool[k];
+        RayState r;
+        int4 h;
+        if (extend_begin<true>(s, pr.o, pr.d, pr.rng1, r, h)) {
+            const int4 b = B.hit[k];
+            r.best.obj = b.x;
+            r.best.prim = b.y;
+            r.best.t = fbits(b.z);
+            h = extend_end<true>(s, pr, r, medium_key);
+        }
+        B.hit[k] = h;
+        bucket_append(ctl->shade_count, B.qsh, B.capacity, hit_model(s, h.x) + 1, k);
+    }
 }
 
 // ------------------------------------------------------------------ shade
@@ -368,6 +399,7 @@ struct ShadowIO {
     const float* pend3;       // four-wavelength mode: pending radiance of wavelength 3
     int spec4;
     unsigned long long traced;
+    int32_t* state;           // kExt: per segment 0 open, 1 blocked, 2 too short, for k_shadow_finish
     __device__ __forceinline__ void finish(int m, bool occ, float tr = 1.0f)
     {
         const float4 dst = rec[m].dst;
@@ -400,23 +432,20 @@ struct ShadowIO {
             ++traced;
             return m;
         }
-        finish(m, false);
+        if (kExt) state[m] = 2;
+        else finish(m, false);
         return -1;
     }
-    __device__ __forceinline__ void store(const SceneView& s, int m, const RayState& r)
+    __device__ __forceinline__ void store(const SceneView&, int m, const RayState& r)
     {
-        float tr;
-        const bool occ = shadow_end<kExt>(s, r, rec[m].src.w, static_cast<uint32_t>(ibits(rec[m].nee.w)), tr);
-        finish(m, occ, tr);
+        if (kExt) state[m] = r.best.obj >= 0 ? 1 : 0;
+        else finish(m, r.best.obj >= 0);
     }
 };
 
 template <bool kExt>
-__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_shadow(SceneView s, PathBuffers B, int cur, PoolCtl* ctl,
-                                                        unsigned long long* stats, uint32_t* ovf, int* err, int spec4)
+__device__ __forceinline__ ShadowIO<kExt> shadow_io(const PathBuffers& B, int cur, int spec4)
 {
-    extern __shared__ uint32_t smem[];
-    const int n = ctl->shadow_count;
     ShadowIO<kExt> io;
     io.rec = B.shadow;
     io.next_pool = pool_of(B, 1 - cur);
@@ -425,11 +454,42 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_shadow(SceneVi
     io.pend3 = B.shadow3;
     io.spec4 = spec4;
     io.traced = 0;
+    io.state = B.qsh;   // the shading queues are free by now
+    return io;
+}
+
+template <bool kExt>
+__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_shadow(SceneView s, PathBuffers B, int cur, PoolCtl* ctl,
+                                                        unsigned long long* stats, uint32_t* ovf, int* err, int spec4)
+{
+    extern __shared__ uint32_t smem[];
+    const int n = ctl->shadow_count;
+    ShadowIO<kExt> io = shadow_io<kExt>(B, cur, spec4);
     traverse_queue<true>(s, io, n, &ctl->fetch_shadow, lane_stack(smem), thread_overflow(ovf), err, &stats[4]);
     unsigned long long c = io.traced;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
     if (lane_id() == 0 && c) atomicAdd(&stats[1], c);
+}
+
+// The rest of a shadow query in scenes with SDF objects or a medium: SDF
+// objects, transmittance, and the light sample's term (see k_extend_finish).
+__global__ void __launch_bounds__(kTraceBlock) k_shadow_finish(SceneView s, PathBuffers B, int cur, PoolCtl* ctl, int spec4)
+{
+    ShadowIO<true> io = shadow_io<true>(B, cur, spec4);
+    const int n = ctl->shadow_count;
+    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += gridDim.x * blockDim.x) {
+        const int st = B.qsh[m];
+        bool occ = st == 1;
+        float tr = 1.0f;
+        if (st == 0) {
+            RayState r;
+            const float4 src = B.shadow[m].src;
+            shadow_begin(src, xyz(B.shadow[m].dst), r);
+            occ = shadow_end<true>(s, r, src.w, static_cast<uint32_t>(ibits(B.shadow[m].nee.w)), tr);
+        }
+        io.finish(m, occ, tr);
+    }
 }
 
 // ------------------------------------------------------------------ retire
@@ -552,8 +612,12 @@ cudaError_t launch_iterations(const SceneView& s, const FrameParams& fp, const P
         launch_generate(fp, B, ctl, b0, b1, jump_table, rec, c, grid_other, st);
         const bool te = tm && tm->n_extend < tm->cap;
         if (te) cudaEventRecord(tm->extend_ev[2 * tm->n_extend], st);
-        if (ext) k_extend<true><<<grid_trace, kTraceBlock, kTraceSmem, st>>>(s, B, c, ctl, stats, ovf, err, fp.medium_key);
-        else k_extend<false><<<grid_trace, kTraceBlock, kTraceSmem, st>>>(s, B, c, ctl, stats, ovf, err, fp.medium_key);
+        if (ext) {
+            k_extend<true><<<grid_trace, kTraceBlock, kTraceSmem, st>>>(s, B, c, ctl, stats, ovf, err);
+            k_extend_finish<<<grid_trace, kTraceBlock, 0, st>>>(s, B, c, ctl, fp.medium_key);
+        } else {
+            k_extend<false><<<grid_trace, kTraceBlock, kTraceSmem, st>>>(s, B, c, ctl, stats, ovf, err);
+        }
         if (te) cudaEventRecord(tm->extend_ev[2 * tm->n_extend++ + 1], st);
         if (fp.spectral == 4 && fp.nrc.enabled) {
             if (ext) launch_shade<true, 4, true>(s, fp, B, c, ctl, rec, grid_other, st);
@@ -577,11 +641,13 @@ cudaError_t launch_iterations(const SceneView& s, const FrameParams& fp, const P
         const bool ts = tm && tm->n_shadow < tm->cap;
         if (ts) cudaEventRecord(tm->shadow_ev[2 * tm->n_shadow], st);
         const int spec4 = fp.spectral == 4 ? 1 : 0;
-        if (ext) k_shadow<true><<<grid_trace, kTraceBlock, kTraceSmem, st>>>(s, B, c, ctl, stats, ovf, err, spec4);
-        else k_shadow<false><<<grid_trace, kTraceBlock, kTraceSmem, st>>>(s, B, c, ctl, stats, ovf, err, spec4);
+        if (ext) {
+            k_shadow<true><<<grid_trace, kTraceBlock, kTraceSmem, st>>>(s, B, c, ctl, stats, ovf, err, spec4);
+            k_shadow_finish<<<grid_trace, kTraceBlock, 0, st>>>(s, B, c, ctl, spec4);
+        } else k_shadow<false><<<grid_trace, kTraceBlock, kTraceSmem, st>>>(s, B, c, ctl, stats, ovf, err, spec4);
         if (ts) cudaEventRecord(tm->shadow_ev[2 * tm->n_shadow++ + 1], st);
         k_retire<<<grid_other, kShadeBlock, 0, st>>>(fp, B, ctl, accum, rec);
-        *launches += s.has_medium ? 11 : 10;
+        *launches += 10 + (ext ? 2 : 0) + (s.has_medium ? 1 : 0);
         *cur = 1 - c;
     }
     return cudaGetLastError();

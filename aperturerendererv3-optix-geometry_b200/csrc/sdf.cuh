@@ -116,7 +116,8 @@ AR_HD m3 m3_of(const float* m)
 
 // Sphere-traced hit distance along the normalised local ray, or -1.  eps_isect
 // is INTERSECT_EPS(depth) of the query; SDF_EPS = eps_isect / 2 (config.cuh:73).
-AR_HD float sdf_march(const SdfRec& g, const Analytic& an, f3 ro, f3 rd, float eps_isect)
+// A caller that drops hits beyond t_max passes it: the march ends there.
+AR_HD float sdf_march(const SdfRec& g, const Analytic& an, f3 ro, f3 rd, float eps_isect, float t_max = INFINITY)
 {
     const f3 c = mk(an.center[0], an.center[1], an.center[2]);
     const f3 e = mk(an.extent[0], an.extent[1], an.extent[2]);
@@ -129,7 +130,7 @@ AR_HD float sdf_march(const SdfRec& g, const Analytic& an, f3 ro, f3 rd, float e
     const f3 tmn = vmin(t1, t2), tmx = vmax(t1, t2);
     const float tEnter = fmaxf(fmaxf(tmn.x, tmn.y), tmn.z);
     const float tExit = fminf(fminf(tmx.x, tmx.y), tmx.z);
-    if (tEnter > tExit || tExit <= 0.0f) return -1.0f;
+    if (tEnter > tExit || tExit <= 0.0f || tEnter > t_max) return -1.0f;
     const float eps = eps_isect * 0.5f;
     const float minStep = eps * 0.5f;
     const float scale = g.kind == kSdfVolume ? kSdfVolumeStepScale : 1.0f;
@@ -143,7 +144,7 @@ AR_HD float sdf_march(const SdfRec& g, const Analytic& an, f3 ro, f3 rd, float e
         if (startInside ? (dLocal > 0.0f && dLocal < eps) : (dLocal < 0.0f && -dLocal < eps)) return tLast;
         const float adv = g.kind == kSdfVolume ? fmaxf(fabsf(dLocal) * scale, minStep) : fmaxf(fabsf(dLocal), minStep);
         t += adv;
-        if (t > tExit) break;
+        if (t > tExit || t > t_max) break;
     }
     return -1.0f;
 }

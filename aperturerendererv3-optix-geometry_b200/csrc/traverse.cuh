@@ -177,7 +177,7 @@ static __device__ __noinline__ void sdf_closest(const SceneView& s, f3 o, f3 d, 
 {
     for (int k = 0; k < s.num_sdf; ++k) {
         const SdfRec g = s.sdf[k];
-        const float t = sdf_march(g, s.analytic[g.analytic], o, d, eps);
+        const float t = sdf_march(g, s.analytic[g.analytic], o, d, eps, *best_t);
         if (t < 0.0f || t < tmin) continue;
         if (t < *best_t || (t == *best_t && *best_obj >= 0 && g.object < *best_obj)) {
             *best_t = t;
@@ -191,7 +191,7 @@ static __device__ __noinline__ int32_t sdf_any(const SceneView& s, f3 o, f3 d, f
 {
     for (int k = 0; k < s.num_sdf; ++k) {
         const SdfRec g = s.sdf[k];
-        const float t = sdf_march(g, s.analytic[g.analytic], o, d, eps);
+        const float t = sdf_march(g, s.analytic[g.analytic], o, d, eps, tmax);
         if (t >= 0.0f && !(t < tmin) && t < tmax) return g.object;
     }
     return -1;
