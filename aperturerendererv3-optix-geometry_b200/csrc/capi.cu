@@ -123,6 +123,8 @@ struct ar_scene {
     float4* spec_lut_lam = nullptr;
     float4* spec_lut_rgb = nullptr;
     int spec_res = 0;
+    float4* spec_basis = nullptr;               // material_basis entries (update_basis)
+    int num_materials = 0;
     void* medium_grid = nullptr;                // density grid of the participating medium
     float bounds[6] = {0, 0, 0, 0, 0, 0};       // box of the BVH root (min xyz, max xyz)
     std::vector<ar::SdfRec> h_sdf;              // data pointers into h_volumes
@@ -303,6 +305,8 @@ ar::FrameParams make_frame(const ar_scene* s, const ar_camera* c, const ar_rende
             fp.spec.lut_lam = s->spec_lut_lam;
             fp.spec.lut_rgb = s->spec_lut_rgb;
             fp.spec.res = s->spec_res;
+            fp.spec.basis = s->spec_basis;
+            fp.spec.materials = s->num_materials;
         }
     }
     for (int d = 0; d <= 8; ++d) fp.eps_tab[d] = 1.0e-3f * exp_det(fminf(static_cast<float>(d) * 0.5f, 4.0f));
@@ -437,6 +441,15 @@ ar_status run_render(ar_scene* s, const ar_camera* cam, const ar_render_params* 
         stats->shadow_ms = s_ms;
     }
     return AR_OK;
+}
+
+// The spectral bases of the scene's materials and medium; after a change of the
+// lookup table or the medium.
+void update_basis(ar_scene* s)
+{
+    if (!s->spec_basis) return;
+    ck(ar::launch_material_basis(s->view.materials, s->num_materials, s->view.medium.albedo, s->spec_lut_rgb, s->spec_res,
+                                 s->spec_basis, nullptr), "spectral material table");
 }
 
 ar_status check_err(ar_scene* s, cudaStream_t st)
@@ -574,6 +587,7 @@ ar_status ar_scene_create_ex(const ar_object_desc* objects, size_t count, const 
         s->objects = static_cast<int64_t>(count);
         s->triangles = hs.triangles;
         s->lights = static_cast<int64_t>(hs.light_object.size());
+        s->num_materials = static_cast<int>(hs.materials.size());
         s->nodes = static_cast<int64_t>(hs.nodes.size());
         s->prims = static_cast<int64_t>(hs.prims.size());
         s->h_objects = std::move(hs.objects);
@@ -715,8 +729,9 @@ ar_status ar_scene_set_spectral_ex(ar_scene* s, const float* tables, size_t coun
             if (*it == p) { s->owned.erase(it); break; }
         cudaFree(p);
     };
-    drop(s->spec_tables); drop(s->spec_lut_lam); drop(s->spec_lut_rgb);
+    drop(s->spec_tables); drop(s->spec_lut_lam); drop(s->spec_lut_rgb); drop(s->spec_basis);
     s->spec_tables = nullptr; s->spec_lut_lam = nullptr; s->spec_lut_rgb = nullptr; s->spec_res = 0;
+    s->spec_basis = nullptr;
     const size_t nrgb = static_cast<size_t>(lut_res) * lut_res * lut_res;
     float* tab = dalloc<float>(count, "spectral tables");
     s->owned.push_back(tab);
@@ -736,11 +751,15 @@ ar_status ar_scene_set_spectral_ex(ar_scene* s, const float* tables, size_t coun
         ck(e, "spectral rgb table on the tensor cores");
         if (h) return fail(AR_ERR_DEVICE_FAULT, "tensor-core table build: an MMA did not complete within its wait limit");
     }
+    float4* basis = dalloc<float4>(static_cast<size_t>(s->num_materials + 1) * ar::kBasisWords, "spectral material table");
+    s->owned.push_back(basis);
+    s->spec_lut_rgb = rgb;
+    s->spec_res = lut_res;
+    s->spec_basis = basis;
+    update_basis(s);
     ck(cudaDeviceSynchronize(), "spectral tables");
     s->spec_tables = tab;
     s->spec_lut_lam = lam;
-    s->spec_lut_rgb = rgb;
-    s->spec_res = lut_res;
     return AR_OK;
     AR_GUARD_END
 }
@@ -801,6 +820,8 @@ ar_status ar_scene_set_medium(ar_scene* s, const ar_medium_desc* m)
     r.fp16 = m->precision == 16 ? 1 : 0;
     r.data = grid;
     s->view.has_medium = 1;
+    update_basis(s);
+    ck(cudaStreamSynchronize(nullptr), "medium");
     return AR_OK;
     AR_GUARD_END
 }

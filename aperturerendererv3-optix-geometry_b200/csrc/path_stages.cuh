@@ -146,11 +146,11 @@ __device__ __forceinline__ int hit_model(const SceneView& s, int obj)
 
 // ------------------------------------------------------------------ shade
 // G-buffer of an RGB material at one wavelength (EvaluateMaterial, spectral).
-__device__ __forceinline__ GB gb_at(const GB& rgb, const SpectralView& sv, const float4& lk, float lambda)
+__device__ __forceinline__ GB gb_at(const GB& rgb, const MaterialBasis& mb, const float4& lk, float lambda)
 {
     GB g = rgb;
-    const float a = interact(sv.lut_rgb, sv.res, lk, rgb.albedo);
-    const float e = interact(sv.lut_rgb, sv.res, lk, rgb.emissive);
+    const float a = interact(mb.albedo, lk);
+    const float e = interact(mb.emissive, lk);
     g.albedo = mk(a, a, a);
     g.emissive = mk(e, e, e);
     g.ior = ior_abbe(lambda, rgb.ior, rgb.abbe);
@@ -283,19 +283,15 @@ __device__ __forceinline__ void shade_path(const SceneView& s, const FrameParams
     // ---- intersection details (re-run of the accepted test)
     f3 pos = mk(0.0f, 0.0f, 0.0f), nrm = mk(0.0f, 0.0f, 0.0f);
     GB gb, gbr;
+    MaterialBasis mb;   // spectral: of the hit's material
     int light = -1;
     if (hit) {
         const ObjInfo oi = s.objects[hr.x];
         gb = load_gb(s.materials[oi.material]);
         gbr = gb;
         if (kSpec) {  // EvaluateMaterial / SampleBSDF at the path's wavelength (material.cuh)
-            const float a = interact(fp.spec.lut_rgb, fp.spec.res, lk, gb.albedo);
-            const float e = interact(fp.spec.lut_rgb, fp.spec.res, lk, gb.emissive);
-            gb.albedo = mk(a, a, a);
-            gb.emissive = mk(e, e, e);
-            gb.ior = ior_abbe(lambda, gb.ior, gb.abbe);
-            gb.sigma_a = sigma_tilt(gb.sigma_a, lambda, gb.tilt);
-            gb.spectral = true;
+            mb = material_basis(fp.spec.basis, oi.material);
+            gb = gb_at(gbr, mb, lk, lambda);
         }
         light = oi.light;
         if (oi.type == AR_OBJ_TRIANGLE) {
@@ -452,10 +448,8 @@ __device__ __forceinline__ void shade_path(const SceneView& s, const FrameParams
         brdf = eval_bsdf_cos(model, crd, next, N, pos, gb, inside, vloc);
         if (kSpec == 4) {
             if (model != AR_MAT_GLASS) {
-                emis = mk(interact(fp.spec.lut_rgb, fp.spec.res, lk4[0], gbr.emissive),
-                          interact(fp.spec.lut_rgb, fp.spec.res, lk4[1], gbr.emissive),
-                          interact(fp.spec.lut_rgb, fp.spec.res, lk4[2], gbr.emissive));
-                emis3 = interact(fp.spec.lut_rgb, fp.spec.res, lk4[3], gbr.emissive);
+                emis = mk(interact(mb.emissive, lk4[0]), interact(mb.emissive, lk4[1]), interact(mb.emissive, lk4[2]));
+                emis3 = interact(mb.emissive, lk4[3]);
             }
             if (model == AR_MAT_GLASS && gbr.abbe > 0.0f && !(flags & kFlagHeroOnly)) {
                 // dispersive glass: the other wavelengths cannot follow the hero's
@@ -463,9 +457,9 @@ __device__ __forceinline__ void shade_path(const SceneView& s, const FrameParams
                 // becomes that of a single-wavelength sample)
                 dispersed = true;
             } else if (model != AR_MAT_LIGHT && !(flags & kFlagHeroOnly)) {
-                const float b1 = eval_bsdf_cos(model, crd, next, N, pos, gb_at(gbr, fp.spec, lk4[1], lam4[1]), inside, vloc).x;
-                const float b2 = eval_bsdf_cos(model, crd, next, N, pos, gb_at(gbr, fp.spec, lk4[2], lam4[2]), inside, vloc).x;
-                brdf3 = eval_bsdf_cos(model, crd, next, N, pos, gb_at(gbr, fp.spec, lk4[3], lam4[3]), inside, vloc).x;
+                const float b1 = eval_bsdf_cos(model, crd, next, N, pos, gb_at(gbr, mb, lk4[1], lam4[1]), inside, vloc).x;
+                const float b2 = eval_bsdf_cos(model, crd, next, N, pos, gb_at(gbr, mb, lk4[2], lam4[2]), inside, vloc).x;
+                brdf3 = eval_bsdf_cos(model, crd, next, N, pos, gb_at(gbr, mb, lk4[3], lam4[3]), inside, vloc).x;
                 brdf = mk(brdf.x, b1, b2);
             }
         }
@@ -476,13 +470,12 @@ __device__ __forceinline__ void shade_path(const SceneView& s, const FrameParams
         pdf = hg_phase(s.medium.g, dot(crd, next));
         malb = mk(s.medium.albedo[0], s.medium.albedo[1], s.medium.albedo[2]);
         if (kSpec == 4) {
-            const f3 rgb = malb;
-            malb = mk(interact(fp.spec.lut_rgb, fp.spec.res, lk4[0], rgb), interact(fp.spec.lut_rgb, fp.spec.res, lk4[1], rgb),
-                      interact(fp.spec.lut_rgb, fp.spec.res, lk4[2], rgb));
-            malb3 = interact(fp.spec.lut_rgb, fp.spec.res, lk4[3], rgb);
+            const RgbBasis ab = material_basis(fp.spec.basis, fp.spec.materials).albedo;
+            malb = mk(interact(ab, lk4[0]), interact(ab, lk4[1]), interact(ab, lk4[2]));
+            malb3 = interact(ab, lk4[3]);
             brdf3 = malb3 * pdf;
         } else if (kSpec) {
-            const float a = interact(fp.spec.lut_rgb, fp.spec.res, lk, malb);
+            const float a = interact(material_basis(fp.spec.basis, fp.spec.materials).albedo, lk);
             malb = mk(a, a, a);
         }
         brdf = malb * pdf;
@@ -496,13 +489,12 @@ __device__ __forceinline__ void shade_path(const SceneView& s, const FrameParams
         pdf = 1.0f;
         emis = sky_lighting(crd, fp.sky);
         if (kSpec == 4) {
-            const f3 rgb = emis;
-            emis = mk(interact(fp.spec.lut_rgb, fp.spec.res, lk4[0], rgb), interact(fp.spec.lut_rgb, fp.spec.res, lk4[1], rgb),
-                      interact(fp.spec.lut_rgb, fp.spec.res, lk4[2], rgb));
-            emis3 = interact(fp.spec.lut_rgb, fp.spec.res, lk4[3], rgb);
+            const RgbBasis eb = rgb_basis(fp.spec.lut_rgb, fp.spec.res, emis);
+            emis = mk(interact(eb, lk4[0]), interact(eb, lk4[1]), interact(eb, lk4[2]));
+            emis3 = interact(eb, lk4[3]);
             brdf3 = 1.0f;
         } else if (kSpec) {
-            const float e = interact(fp.spec.lut_rgb, fp.spec.res, lk, emis);
+            const float e = interact(rgb_basis(fp.spec.lut_rgb, fp.spec.res, emis), lk);
             emis = mk(e, e, e);
         }
         nInside = false;
@@ -582,9 +574,10 @@ __device__ __forceinline__ void shade_path(const SceneView& s, const FrameParams
             const float rate = sqrtf(saturate(lum));
             if (fp.use_nee && nonDelta < 10 && !delta && !mInside && g.next() < rate) {
                 LightSample ls = sample_light(s, pos, g, fp.tri_light_nee != 0);
-                const f3 lsRgb = ls.emis;
-                if (kSpec) {
-                    const float e = interact(fp.spec.lut_rgb, fp.spec.res, lk, ls.emis);
+                RgbBasis lb;   // spectral: of the light's emission
+                if (kSpec && ls.valid) {
+                    lb = material_basis(fp.spec.basis, ls.material).emissive;
+                    const float e = interact(lb, lk);
                     ls.emis = mk(e, e, e);
                 }
                 if (ls.valid) {
@@ -618,15 +611,15 @@ __device__ __forceinline__ void shade_path(const SceneView& s, const FrameParams
                                 f1 = malb.y * ph; f2 = malb.z * ph; f3v = malb3 * ph;
                             } else {
                                 const f3 z0 = mk(0.0f, 0.0f, 0.0f);
-                                f1 = eval_bsdf_cos(model, crd, ld, nrm, pos, gb_at(gbr, fp.spec, lk4[1], lam4[1]), false, z0).x;
-                                f2 = eval_bsdf_cos(model, crd, ld, nrm, pos, gb_at(gbr, fp.spec, lk4[2], lam4[2]), false, z0).x;
-                                f3v = eval_bsdf_cos(model, crd, ld, nrm, pos, gb_at(gbr, fp.spec, lk4[3], lam4[3]), false, z0).x;
+                                f1 = eval_bsdf_cos(model, crd, ld, nrm, pos, gb_at(gbr, mb, lk4[1], lam4[1]), false, z0).x;
+                                f2 = eval_bsdf_cos(model, crd, ld, nrm, pos, gb_at(gbr, mb, lk4[2], lam4[2]), false, z0).x;
+                                f3v = eval_bsdf_cos(model, crd, ld, nrm, pos, gb_at(gbr, mb, lk4[3], lam4[3]), false, z0).x;
                             }
                             const f3 c3 = mk(contrib.x,
-                                             (f1 * interact(fp.spec.lut_rgb, fp.spec.res, lk4[1], lsRgb)) * G4,
-                                             (f2 * interact(fp.spec.lut_rgb, fp.spec.res, lk4[2], lsRgb)) * G4);
+                                             (f1 * interact(lb, lk4[1])) * G4,
+                                             (f2 * interact(lb, lk4[2])) * G4);
                             pending = (mask * (c3 * wmis)) * d65v;
-                            pend3 = (mask3 * (((f3v * interact(fp.spec.lut_rgb, fp.spec.res, lk4[3], lsRgb)) * G4) * wmis)) * d65_3;
+                            pend3 = (mask3 * (((f3v * interact(lb, lk4[3])) * G4) * wmis)) * d65_3;
                         }
                     }
                     shadow = true;

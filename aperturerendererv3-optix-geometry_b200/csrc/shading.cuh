@@ -350,6 +350,7 @@ static __device__ float pdf_light_from_hit(const SceneView& s, int obj, f3 sp, f
 struct LightSample {
     f3 p, n, emis;
     float pFacet, pA;
+    int material;
     bool valid;
 };
 
@@ -373,6 +374,7 @@ static __device__ LightSample sample_light(const SceneView& s, f3 sp, Rng& g, bo
     const int lobj = s.light_object[pick];
     const ObjInfo oi = s.objects[lobj];
     const MaterialRec& mr = s.materials[oi.material];
+    ls.material = oi.material;
     if (oi.type == AR_OBJ_CUBE) {
         const Analytic& an = s.analytic[oi.aux];
         Box6 b;

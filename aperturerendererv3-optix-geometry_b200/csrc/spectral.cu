@@ -42,7 +42,29 @@ __global__ void __launch_bounds__(128) k_lut_rgb(const float* __restrict__ tab, 
     }
 }
 
+// material_basis entries of `count` materials and, last, of the medium's albedo
+__global__ void k_material_basis(const MaterialRec* __restrict__ mats, int count, f3 medium, const float4* __restrict__ lut,
+                                 int res, float4* __restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > count) return;
+    const f3 a = i < count ? mk(mats[i].albedo[0], mats[i].albedo[1], mats[i].albedo[2]) : medium;
+    const f3 e = i < count ? mk(mats[i].emissive[0], mats[i].emissive[1], mats[i].emissive[2]) : mk(0.0f, 0.0f, 0.0f);
+    const RgbBasis ab = rgb_basis(lut, res, a), eb = rgb_basis(lut, res, e);
+    out[kBasisWords * i] = ab.k;
+    out[kBasisWords * i + 1] = eb.k;
+    out[kBasisWords * i + 2] = make_float4(ab.scale, eb.scale, 0.0f, 0.0f);
+}
+
 }  // namespace
+
+cudaError_t launch_material_basis(const MaterialRec* mats, int count, const float* medium_albedo, const float4* lut_rgb, int res,
+                                  float4* out, cudaStream_t st)
+{
+    k_material_basis<<<count / 128 + 1, 128, 0, st>>>(mats, count, mk(medium_albedo[0], medium_albedo[1], medium_albedo[2]),
+                                                      lut_rgb, res, out);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_spectral_luts(const float* tab, int res, float4* lut_lam, float4* lut_rgb, int sm_count,
                                  cudaStream_t st)

@@ -44,8 +44,9 @@ struct SpectralView {
     const float* tables;     // kTabFloats values (device)
     const float4* lut_rgb;   // res^3 entries, x fastest
     const float4* lut_lam;   // kLambdaLutRes entries
+    const float4* basis;     // material_basis entries: the scene's materials, then the medium
     int32_t res;
-    int32_t pad;
+    int32_t materials;       // index of the medium's entry
 };
 
 // ---------------------------------------------------------------- tables
@@ -351,20 +352,52 @@ AR_HD void query_rgb(const float4* lut, int res, f3 rgb, float* k)
     accum4(lut[x1 + y1 * sy + z1 * sz], wx1 * wy1 * wz1, k);
 }
 
-// spectrum::lut::Interact (spectrum_lut.cuh:222-236): reflectance or emission
-// of an RGB colour at the wavelength whose basis is lk; colours above 1 are
-// normalised by their maximum and scaled back.
-AR_HD float interact(const float4* lut, int res, float4 lk, f3 rgb)
+// The part of spectrum::lut::Interact (spectrum_lut.cuh:222-236) that depends on
+// the RGB colour alone: its basis coefficients, and the factor by which colours
+// above 1 are normalised and scaled back.
+struct RgbBasis {
+    float4 k;
+    float scale;
+};
+AR_HD RgbBasis rgb_basis(const float4* lut, int res, f3 rgb)
 {
     const float lum = fmaxf(rgb.x, fmaxf(rgb.y, rgb.z));
     float k[4];
-    const float l4[4] = {lk.x, lk.y, lk.z, lk.w};
+    RgbBasis b;
+    b.scale = 1.0f;
     if (lum > 1.0f) {
         query_rgb(lut, res, mk(rgb.x / lum, rgb.y / lum, rgb.z / lum), k);
-        return spectral_interact(k, l4) * lum;
+        b.scale = lum;
+    } else {
+        query_rgb(lut, res, rgb, k);
     }
-    query_rgb(lut, res, rgb, k);
-    return spectral_interact(k, l4);
+    b.k = make_float4(k[0], k[1], k[2], k[3]);
+    return b;
+}
+
+// Interact: reflectance or emission of the colour at the wavelength whose basis is lk.
+AR_HD float interact(const RgbBasis& b, const float4& lk)
+{
+    const float k[4] = {b.k.x, b.k.y, b.k.z, b.k.w}, l4[4] = {lk.x, lk.y, lk.z, lk.w};
+    return spectral_interact(k, l4) * b.scale;
+}
+
+// Per material: bases of its albedo and emission (three float4 in
+// SpectralView::basis: albedo, emission, the two scales); after the last
+// material one entry for the medium's single-scattering albedo.
+struct MaterialBasis {
+    RgbBasis albedo, emissive;
+};
+constexpr int kBasisWords = 3;   // float4 per entry
+AR_HD MaterialBasis material_basis(const float4* basis, int entry)
+{
+    const float4 a = basis[kBasisWords * entry], e = basis[kBasisWords * entry + 1], c = basis[kBasisWords * entry + 2];
+    MaterialBasis b;
+    b.albedo.k = a;
+    b.albedo.scale = c.x;
+    b.emissive.k = e;
+    b.emissive.scale = c.y;
+    return b;
 }
 
 }  // namespace ar
