@@ -103,6 +103,51 @@ constexpr int64_t kMaxPool = int64_t(1) << 21;  // paths in flight
 // of its resident blocks.
 int tail_limit(int sm_count) { return ar::kTailBlocks * sm_count * ar::kTraceBlock; }
 
+// What a batch needs besides its graph, kept by the scene of its first job from
+// one batch to the next: the jobs' workspaces as one allocation (at most
+// kBatchKeep bytes are kept), and a stream and an event per job.  A second batch
+// that runs at the same time finds the lock taken and makes its own.
+constexpr size_t kBatchKeep = size_t(4) << 30;
+struct BatchArena {
+    std::mutex lock;
+    char* mem = nullptr;
+    size_t bytes = 0;
+    std::vector<cudaStream_t> streams;
+    std::vector<cudaEvent_t> events;
+    void clear()
+    {
+        if (mem) cudaFree(mem);
+        mem = nullptr;
+        bytes = 0;
+        for (cudaEvent_t e : events) cudaEventDestroy(e);
+        for (cudaStream_t s : streams) cudaStreamDestroy(s);
+        events.clear();
+        streams.clear();
+    }
+    void reserve(size_t need)
+    {
+        if (bytes >= need) return;
+        if (mem) cudaFree(mem);
+        mem = nullptr;
+        bytes = 0;
+        mem = dalloc<char>(need, "batch workspaces");
+        bytes = need;
+    }
+    void handles(size_t n)
+    {
+        while (streams.size() < n) {
+            cudaStream_t s;
+            ck(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
+            streams.push_back(s);
+        }
+        while (events.size() < n) {
+            cudaEvent_t e;
+            ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+            events.push_back(e);
+        }
+    }
+};
+
 }  // namespace
 
 struct ar_scene {
@@ -149,6 +194,7 @@ struct ar_scene {
     int* err = nullptr;
     uint32_t* ovf = nullptr;  // traversal stack overflow slabs, one per persistent thread
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    BatchArena batch;   // of batches whose first job is this scene's
     std::vector<cudaEvent_t> timer_ext, timer_sh;  // event pairs around traversal launches
 
     ~ar_scene()
@@ -156,6 +202,7 @@ struct ar_scene {
         QuietDeviceGuard g(device);
         for (void* p : owned) cudaFree(p);
         if (ws) cudaFree(ws);
+        batch.clear();
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         for (cudaEvent_t e : timer_ext) cudaEventDestroy(e);
@@ -848,7 +895,6 @@ namespace {
 
 // Workspace of one job of a batch (the same layout as a scene's own).
 struct JobWs {
-    char* mem = nullptr;
     ar::PathBuffers B{};
     uint4* base0 = nullptr;
     uint2* base1 = nullptr;
@@ -864,7 +910,8 @@ struct JobWs {
     int cur = 0;
 };
 
-void job_alloc(JobWs& w, int64_t pool, int64_t npix, int grid_trace)
+// Lays the workspace out at b; returns its size (b may be NULL to ask for it).
+size_t job_layout(JobWs& w, char* b, int64_t pool, int64_t npix, int grid_trace)
 {
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
@@ -876,8 +923,7 @@ void job_alloc(JobWs& w, int64_t pool, int64_t npix, int grid_trace)
     const size_t o_b0 = take(16 * N), o_b1 = take(8 * N), o_acc = take(24 * N);
     const size_t o_cnt = take(sizeof(ar::PoolCtl)), o_stats = take(64), o_err = take(64);
     const size_t o_ovf = take(static_cast<size_t>(grid_trace) * ar::kTraceBlock * ar::kStackOverflow * 4);
-    w.mem = dalloc<char>(off, "batch job workspace");
-    char* b = w.mem;
+    if (!b) return off;
     w.B.pool[0] = reinterpret_cast<ar::PathRec*>(b + o_p0);
     w.B.pool[1] = reinterpret_cast<ar::PathRec*>(b + o_p1);
     w.B.hit = reinterpret_cast<int4*>(b + o_hit);
@@ -895,6 +941,7 @@ void job_alloc(JobWs& w, int64_t pool, int64_t npix, int grid_trace)
     w.stats = reinterpret_cast<unsigned long long*>(b + o_stats);
     w.err = reinterpret_cast<int*>(b + o_err);
     w.ovf = reinterpret_cast<uint32_t*>(b + o_ovf);
+    return off;
 }
 
 // Device-side end test of the batch loop: after each pass of the loop body
@@ -928,23 +975,31 @@ __global__ void k_batch_drain(BatchDrain d, cudaGraphConditionalHandle h)
 
 struct BatchResources {
     std::vector<JobWs> jobs;
-    void* drain_mem = nullptr;      // BatchDrain tables and counters
+    BatchArena own;                 // used when the scene's arena is taken
+    BatchArena* arena = nullptr;
+    std::unique_lock<std::mutex> held;
     cudaEvent_t fork = nullptr;
     cudaStream_t orch = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    bool capturing = false;         // orch captures into the graph's loop body
     ~BatchResources()
     {
+        if (capturing) {   // an error while capturing: end it before the graph goes
+            cudaGraph_t g = nullptr;
+            cudaStreamEndCapture(orch, &g);
+            cudaGetLastError();
+        }
+        // also after an error: nothing of the batch may still use the arena
+        if (orch) cudaStreamSynchronize(orch);
+        for (JobWs& w : jobs)
+            if (w.st) cudaStreamSynchronize(w.st);
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
         if (fork) cudaEventDestroy(fork);
-        if (drain_mem) cudaFree(drain_mem);
         if (orch) cudaStreamDestroy(orch);
-        for (JobWs& w : jobs) {
-            if (w.done) cudaEventDestroy(w.done);
-            if (w.st) cudaStreamDestroy(w.st);
-            if (w.mem) cudaFree(w.mem);
-        }
+        own.clear();
+        if (arena && arena != &own && arena->bytes > kBatchKeep) arena->clear();
     }
 };
 
@@ -1035,14 +1090,19 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
     AR_GUARD_BEGIN
     DeviceGuard g(s0->device);
     cudaStream_t user = static_cast<cudaStream_t>(stream);
-    int K = iterations_per_graph > 0 ? iterations_per_graph : 16;
-    K += K & 1;  // even: both pool buffers back in place after a replay
     // In-flight paths: a shared budget split by each job's share of the work
     // (a job never gets more than it has paths, nor fewer than 2^14).
     int64_t totalAll = 0;
     for (int j = 0; j < njobs; ++j)
         totalAll += static_cast<int64_t>(jobs[j].camera.width) * jobs[j].camera.height * jobs[j].params.spp;
     const int64_t budget = path_budget > 0 ? path_budget : (int64_t(1) << 22);
+    // Iterations per pass of the loop: as many as the fullest pool needs to start
+    // all its samples, and some to bring the last paths under the tail's limit
+    // (default; 16 whatever the batch made a graph of 1,900 nodes for 12 stills,
+    // 4.8 ms to instantiate, most of them run with empty pools).
+    int K = iterations_per_graph > 0 ? iterations_per_graph
+                                     : static_cast<int>(std::min<int64_t>(16, (totalAll + budget - 1) / budget + 3));
+    K += K & 1;  // even: both pool buffers back in place after a replay
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     ck(cudaEventCreate(&t0), "event");
     ck(cudaEventCreate(&t1), "event");
@@ -1058,6 +1118,7 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
     ck(cudaStreamWaitEvent(st, R.fork, 0), "order after caller");
     ck(cudaEventRecord(t0, st), "event record");
     ck(cudaEventRecord(R.fork, st), "event record");
+    size_t bytes = 0;
     for (int j = 0; j < njobs; ++j) {
         JobWs& w = R.jobs[j];
         const ar_job& jb = jobs[j];
@@ -1070,9 +1131,20 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
         w.pool = std::max<int64_t>(1, std::min<int64_t>(pool, w.total));
         w.fp = make_frame(jb.scene, &jb.camera, &jb.params);
         w.fp.pool = static_cast<int32_t>(w.pool);
-        job_alloc(w, w.pool, w.npix, jb.scene->grid_trace);
-        ck(cudaStreamCreateWithFlags(&w.st, cudaStreamNonBlocking), "stream");
-        ck(cudaEventCreateWithFlags(&w.done, cudaEventDisableTiming), "event");
+        bytes += job_layout(w, nullptr, w.pool, w.npix, jb.scene->grid_trace);
+    }
+    const size_t drain_bytes = static_cast<size_t>(njobs) * 16 + 64;
+    R.held = std::unique_lock<std::mutex>(jobs[0].scene->batch.lock, std::try_to_lock);
+    R.arena = R.held.owns_lock() ? &jobs[0].scene->batch : &R.own;
+    R.arena->reserve(bytes + drain_bytes);
+    R.arena->handles(static_cast<size_t>(njobs));
+    char* next = R.arena->mem;
+    for (int j = 0; j < njobs; ++j) {
+        JobWs& w = R.jobs[j];
+        const ar_job& jb = jobs[j];
+        next += job_layout(w, next, w.pool, w.npix, jb.scene->grid_trace);
+        w.st = R.arena->streams[static_cast<size_t>(j)];
+        w.done = R.arena->events[static_cast<size_t>(j)];
         ck(cudaStreamWaitEvent(w.st, R.fork, 0), "fork");
         ck(ar::launch_rng_init(w.fp, w.base0, w.base1, jb.scene->init_tables, jb.scene->sm_count, w.st), "rng init");
         ck(ar::launch_render_init(w.ctl, w.total, w.accum, w.npix, w.stats, w.err, jb.scene->sm_count, w.st), "render init");
@@ -1082,31 +1154,24 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
     int64_t maxDepth = 0, maxRatio = 0;
     for (int j = 0; j < njobs; ++j) {
         maxDepth = std::max<int64_t>(maxDepth, jobs[j].params.max_depth);
-        const int64_t admit = std::max<int64_t>(1, std::min<int64_t>(R.jobs[j].pool, R.jobs[j].npix));
-        maxRatio = std::max<int64_t>(maxRatio, R.jobs[j].total / admit + 2);
+        maxRatio = std::max<int64_t>(maxRatio, R.jobs[j].total / R.jobs[j].pool + 2);
     }
     const int64_t maxPasses = (maxRatio * (maxDepth + 2)) / K + 2;
     // The drain test's tables: per job its pool control block and path total.
-    {
-        const size_t nj = static_cast<size_t>(njobs);
-        R.drain_mem = dalloc<unsigned char>(nj * 16 + 64, "batch drain tables");
-        std::vector<const ar::PoolCtl*> ctls(nj);
-        std::vector<int64_t> totals(nj);
-        for (size_t j = 0; j < nj; ++j) {
-            ctls[j] = R.jobs[j].ctl;
-            totals[j] = R.jobs[j].total;
-        }
-        unsigned char* m = static_cast<unsigned char*>(R.drain_mem);
-        ck(cudaMemcpyAsync(m, ctls.data(), nj * 8, cudaMemcpyHostToDevice, st), "drain tables");
-        ck(cudaMemcpyAsync(m + nj * 8, totals.data(), nj * 8, cudaMemcpyHostToDevice, st), "drain tables");
-        ck(cudaMemsetAsync(m + nj * 16, 0, 64, st), "drain counters");
+    const size_t nj = static_cast<size_t>(njobs);
+    std::vector<unsigned char> tab(drain_bytes, 0);
+    for (size_t j = 0; j < nj; ++j) {
+        const ar::PoolCtl* c = R.jobs[j].ctl;
+        std::memcpy(tab.data() + 8 * j, &c, 8);
+        std::memcpy(tab.data() + 8 * (nj + j), &R.jobs[j].total, 8);
     }
+    ck(cudaMemcpyAsync(next, tab.data(), drain_bytes, cudaMemcpyHostToDevice, st), "drain tables");
     BatchDrain dr;
-    dr.ctl = reinterpret_cast<const ar::PoolCtl* const*>(R.drain_mem);
-    dr.total = reinterpret_cast<const int64_t*>(static_cast<unsigned char*>(R.drain_mem) + njobs * 8);
+    dr.ctl = reinterpret_cast<const ar::PoolCtl* const*>(next);
+    dr.total = reinterpret_cast<const int64_t*>(next + nj * 8);
     dr.jobs = njobs;
     dr.max_passes = static_cast<int32_t>(std::min<int64_t>(maxPasses, INT32_MAX));
-    dr.passes = reinterpret_cast<int32_t*>(static_cast<unsigned char*>(R.drain_mem) + njobs * 16);
+    dr.passes = reinterpret_cast<int32_t*>(next + nj * 16);
     // One graph, launched once: a WHILE conditional node whose body runs K
     // wavefront iterations of every job (each job on its own branch) and then
     // the drain test, which sets the node's condition on the device -- no host
@@ -1124,6 +1189,7 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     ck(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
        "begin capture");
+    R.capturing = true;
     ck(cudaEventRecord(R.fork, st), "fork");
     int64_t launches = 0;
     for (int j = 0; j < njobs; ++j) {
@@ -1138,12 +1204,16 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
         ck(ar::launch_iterations(jb.scene->view, w.fp, w.B, w.ctl, w.base0, w.base1, jb.scene->jump_table, w.stats,
                                  w.ovf, w.err, w.accum, nullptr, K, &w.cur, gt, go, w.st, &launches, nullptr),
            "capture iterations");
+        ck(ar::launch_tail(jb.scene->view, w.fp, w.B, w.ctl, w.stats, w.ovf, w.err, w.accum, nullptr, w.cur,
+                           tail_limit(jb.scene->sm_count), jb.scene->sm_count, w.st), "capture tail");
+        ++launches;
         ck(cudaEventRecord(w.done, w.st), "join");
         ck(cudaStreamWaitEvent(st, w.done, 0), "join");
     }
     k_batch_drain<<<1, 256, 0, st>>>(dr, cond);
     ck(cudaGetLastError(), "drain test");
     cudaGraph_t captured = nullptr;
+    R.capturing = false;
     ck(cudaStreamEndCapture(st, &captured), "end capture");
     ck(cudaGraphInstantiate(&R.exec, R.graph, 0), "graph instantiate");
     size_t nodes = 0;
@@ -1156,20 +1226,22 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
     const int64_t replays = dres[0];
     // outputs, counters, error words
     unsigned long long ext = 0, sh = 0;
-    for (int j = 0; j < njobs; ++j) {
+    std::vector<unsigned long long> h(2 * nj);
+    std::vector<int> errs(nj);
+    for (size_t j = 0; j < nj; ++j) {
         JobWs& w = R.jobs[j];
         const ar_job& jb = jobs[j];
         const int64_t n = w.npix * 3;
         if (jb.out_rgb) ck(ar::launch_mean(w.accum, n, 1.0 / static_cast<double>(jb.params.spp), jb.out_rgb, st), "mean");
         if (jb.accum) ck(ar::launch_add(w.accum, n, jb.accum, st), "accumulate");
-        unsigned long long h[2];
-        int e = 0;
-        ck(cudaMemcpyAsync(h, w.stats, sizeof(h), cudaMemcpyDeviceToHost, st), "stats");
-        ck(cudaMemcpyAsync(&e, w.err, sizeof(int), cudaMemcpyDeviceToHost, st), "error word");
-        ck(cudaStreamSynchronize(st), "sync");
-        if (e != 0) return fail(AR_ERR_DEVICE_FAULT, "job " + std::to_string(j) + ": traversal stack overflow");
-        ext += h[0];
-        sh += h[1];
+        ck(cudaMemcpyAsync(&h[2 * j], w.stats, 2 * sizeof(h[0]), cudaMemcpyDeviceToHost, st), "stats");
+        ck(cudaMemcpyAsync(&errs[j], w.err, sizeof(int), cudaMemcpyDeviceToHost, st), "error word");
+    }
+    ck(cudaStreamSynchronize(st), "sync");
+    for (size_t j = 0; j < nj; ++j) {
+        if (errs[j] != 0) return fail(AR_ERR_DEVICE_FAULT, "job " + std::to_string(j) + ": traversal stack overflow");
+        ext += h[2 * j];
+        sh += h[2 * j + 1];
     }
     ck(cudaEventRecord(t1, st), "event record");
     ck(cudaEventSynchronize(t1), "sync");
@@ -1352,6 +1424,9 @@ struct ar_nrc {
     int32_t* counters = nullptr;   // [0] queries, [1] samples, [2..] slot vertex counts
     int slots = 0, sample_cap = 0;
     int* tc_err = nullptr;         // error word of the tcgen05 inference kernel
+    char* io = nullptr;            // device copies of a host call's arrays (nrc_io)
+    size_t io_bytes = 0;
+    std::mutex io_lock;
     int tensor_path = 1;           // inference: 1 tcgen05 (default), 0 mma.sync
     int spectral = 0;              // 0 RGB cache, 4 four-wavelength cache (16 spectral bins)
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -1372,6 +1447,7 @@ struct ar_nrc {
     {
         QuietDeviceGuard g(scene->device);
         for (void* p : owned) cudaFree(p);
+        if (io) cudaFree(io);
         for (cudaEvent_t e : ev)
             if (e) cudaEventDestroy(e);
     }
@@ -1396,6 +1472,50 @@ void nrc_ensure_queries(ar_nrc* c, int64_t n)
     c->queries = nrc_alloc<ar::NrcQuery>(c, static_cast<size_t>(n), "cache queries");
     c->query_cap = n;
 }
+
+// Device space for the arrays of a host-buffer call, kept by the cache from call
+// to call (at most kNrcIoKeep bytes: a larger one goes back at the call's end).
+// A call that finds it in use by another thread allocates its own.
+constexpr size_t kNrcIoKeep = size_t(64) << 20;
+struct NrcIo {
+    ar_nrc* c;
+    std::unique_lock<std::mutex> held;
+    char* own = nullptr;
+    char* mem;
+    size_t used = 0;
+    NrcIo(ar_nrc* cache, size_t bytes) : c(cache), held(cache->io_lock, std::try_to_lock)
+    {
+        if (!held.owns_lock()) {
+            mem = own = dalloc<char>(bytes, "cache call buffers");
+            return;
+        }
+        if (bytes > c->io_bytes) {
+            drop();
+            c->io = dalloc<char>(bytes, "cache call buffers");
+            c->io_bytes = bytes;
+        }
+        mem = c->io;
+    }
+    ~NrcIo()
+    {
+        if (own) cudaFree(own);
+        else if (c->io_bytes > kNrcIoKeep) drop();
+    }
+    template <class T>
+    T* take(size_t count)
+    {
+        T* p = reinterpret_cast<T*>(mem + used);
+        used += padded(count * sizeof(T));
+        return p;
+    }
+    static size_t padded(size_t bytes) { return (bytes + 255) & ~size_t(255); }
+    void drop()
+    {
+        if (c->io) cudaFree(c->io);
+        c->io = nullptr;
+        c->io_bytes = 0;
+    }
+};
 
 cudaError_t nrc_run_infer(ar_nrc* c, const ar::NrcQuery* q, const int32_t* count, int cap, double* accum,
                           float* out_rgb, cudaStream_t st)
@@ -1645,29 +1765,21 @@ ar_status ar_nrc_infer(ar_nrc* c, const float* vertices, size_t n, float* out_rg
     if (n == 0) return AR_OK;
     AR_GUARD_BEGIN
     DeviceGuard g(c->scene->device);
-    ar::NrcQuery* q = dalloc<ar::NrcQuery>(n, "queries");
-    float* out = nullptr;
-    int32_t* cnt = nullptr;
-    cudaError_t e = cudaSuccess;
-    try {
-        out = dalloc<float>(n * (c->spectral ? ar::kNrcBins : 3), "predictions");
-        cnt = dalloc<int32_t>(1, "count");
-        std::vector<ar::NrcQuery> h(n);
-        for (size_t i = 0; i < n; ++i) {
-            std::memcpy(&h[i].v, vertices + 16 * i, sizeof(ar::NrcVertex));
-            h[i].t = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-        }
-        const int32_t ni = static_cast<int32_t>(n);
-        ck(cudaMemcpy(q, h.data(), n * sizeof(ar::NrcQuery), cudaMemcpyHostToDevice), "copy vertices");
-        ck(cudaMemcpy(cnt, &ni, 4, cudaMemcpyHostToDevice), "copy count");
-        e = nrc_run_infer(c, q, cnt, ni, nullptr, out, nullptr);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(out_rgb, out, n * 4 * (c->spectral ? ar::kNrcBins : 3), cudaMemcpyDeviceToHost);
-    } catch (...) {
-        cudaFree(q); cudaFree(out); cudaFree(cnt);
-        throw;
+    const size_t outs = n * (c->spectral ? ar::kNrcBins : 3);
+    NrcIo io(c, NrcIo::padded(n * sizeof(ar::NrcQuery)) + NrcIo::padded(outs * 4) + 256);
+    ar::NrcQuery* q = io.take<ar::NrcQuery>(n);
+    float* out = io.take<float>(outs);
+    int32_t* cnt = io.take<int32_t>(1);
+    std::vector<ar::NrcQuery> h(n);
+    for (size_t i = 0; i < n; ++i) {
+        std::memcpy(&h[i].v, vertices + 16 * i, sizeof(ar::NrcVertex));
+        h[i].t = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     }
-    cudaFree(q); cudaFree(out); cudaFree(cnt);
+    const int32_t ni = static_cast<int32_t>(n);
+    ck(cudaMemcpy(q, h.data(), n * sizeof(ar::NrcQuery), cudaMemcpyHostToDevice), "copy vertices");
+    ck(cudaMemcpy(cnt, &ni, 4, cudaMemcpyHostToDevice), "copy count");
+    cudaError_t e = nrc_run_infer(c, q, cnt, ni, nullptr, out, nullptr);
+    if (e == cudaSuccess) e = cudaMemcpy(out_rgb, out, outs * 4, cudaMemcpyDeviceToHost);
     ck(e, "cache inference");
     return nrc_check(c, nullptr);
     AR_GUARD_END
@@ -1681,32 +1793,25 @@ ar_status ar_nrc_gradients(ar_nrc* c, const float* samples, size_t n, float* tab
     if (n > static_cast<size_t>(c->cfg.train_batch)) return fail(AR_ERR_INVALID_ARGUMENT, "n exceeds train_batch");
     AR_GUARD_BEGIN
     DeviceGuard g(c->scene->device);
-    ar::NrcSample* d = dalloc<ar::NrcSample>(n, "samples");
-    int32_t* cnt = nullptr;
-    try {
-        cnt = dalloc<int32_t>(1, "count");
-        const int32_t ni = static_cast<int32_t>(n);
-        ck(cudaMemcpy(d, samples, n * sizeof(ar::NrcSample), cudaMemcpyHostToDevice), "copy samples");
-        ck(cudaMemcpy(cnt, &ni, 4, cudaMemcpyHostToDevice), "copy count");
-        ck(cudaMemset(c->T.loss, 0, 4), "memset");
-        ck(ar::nrc_train_step(c->net(), c->P, d, cnt, 0, c->cfg.train_batch, c->T, c->cfg.learning_rate, c->step + 1,
-                              c->scene->sm_count, nullptr, false, c->tensor_path ? c->tc_err : nullptr),
-           "cache gradients");
-        const size_t tf = static_cast<size_t>(c->P.table_floats);
-        std::vector<float> tg(tf), wg(ar::kNrcParams);
-        ck(cudaMemcpy(tg.data(), c->P.table_g, tf * 4, cudaMemcpyDeviceToHost), "copy gradients");
-        ck(cudaMemcpy(wg.data(), c->P.w_g, ar::kNrcParams * 4, cudaMemcpyDeviceToHost), "copy gradients");
-        if (loss) ck(cudaMemcpy(loss, c->T.loss, 4, cudaMemcpyDeviceToHost), "copy loss");
-        ck(cudaMemset(c->P.table_g, 0, tf * 4), "memset");
-        ck(cudaMemset(c->P.w_g, 0, ar::kNrcParams * 4), "memset");
-        const float inv = 1.0f / ar::kNrcLossScale;
-        if (table_grad) for (size_t i = 0; i < tf; ++i) table_grad[i] = tg[i] * inv;
-        if (weight_grad) for (int i = 0; i < ar::kNrcParams; ++i) weight_grad[i] = wg[static_cast<size_t>(i)] * inv;
-    } catch (...) {
-        cudaFree(d); cudaFree(cnt);
-        throw;
-    }
-    cudaFree(d); cudaFree(cnt);
+    NrcIo io(c, NrcIo::padded(n * sizeof(ar::NrcSample)) + 256);
+    ar::NrcSample* d = io.take<ar::NrcSample>(n);
+    int32_t* cnt = io.take<int32_t>(1);
+    const int32_t ni = static_cast<int32_t>(n);
+    ck(cudaMemcpy(d, samples, n * sizeof(ar::NrcSample), cudaMemcpyHostToDevice), "copy samples");
+    ck(cudaMemcpy(cnt, &ni, 4, cudaMemcpyHostToDevice), "copy count");
+    ck(cudaMemset(c->T.loss, 0, 4), "memset");
+    ck(ar::nrc_train_step(c->net(), c->P, d, cnt, 0, c->cfg.train_batch, c->T, c->cfg.learning_rate, c->step + 1,
+                          c->scene->sm_count, nullptr, false, c->tensor_path ? c->tc_err : nullptr),
+       "cache gradients");
+    const size_t tf = static_cast<size_t>(c->P.table_floats);
+    if (table_grad) ck(cudaMemcpy(table_grad, c->P.table_g, tf * 4, cudaMemcpyDeviceToHost), "copy gradients");
+    if (weight_grad) ck(cudaMemcpy(weight_grad, c->P.w_g, ar::kNrcParams * 4, cudaMemcpyDeviceToHost), "copy gradients");
+    if (loss) ck(cudaMemcpy(loss, c->T.loss, 4, cudaMemcpyDeviceToHost), "copy loss");
+    ck(cudaMemset(c->P.table_g, 0, tf * 4), "memset");
+    ck(cudaMemset(c->P.w_g, 0, ar::kNrcParams * 4), "memset");
+    const float inv = 1.0f / ar::kNrcLossScale;
+    if (table_grad) for (size_t i = 0; i < tf; ++i) table_grad[i] *= inv;
+    if (weight_grad) for (int i = 0; i < ar::kNrcParams; ++i) weight_grad[i] *= inv;
     return nrc_check(c, nullptr);
     AR_GUARD_END
 }
@@ -1718,27 +1823,21 @@ ar_status ar_nrc_train(ar_nrc* c, const float* samples, size_t n, int32_t steps,
     if (n > static_cast<size_t>(INT32_MAX)) return fail(AR_ERR_INVALID_ARGUMENT, "too many samples");
     AR_GUARD_BEGIN
     DeviceGuard g(c->scene->device);
-    ar::NrcSample* d = dalloc<ar::NrcSample>(std::max<size_t>(n, 1), "samples");
-    int32_t* cnt = nullptr;
-    try {
-        cnt = dalloc<int32_t>(1, "count");
-        const int32_t ni = static_cast<int32_t>(n);
-        if (n) ck(cudaMemcpy(d, samples, n * sizeof(ar::NrcSample), cudaMemcpyHostToDevice), "copy samples");
-        ck(cudaMemcpy(cnt, &ni, 4, cudaMemcpyHostToDevice), "copy count");
-        for (int k = 0; k < steps; ++k) {
-            ck(cudaMemset(c->T.loss, 0, 4), "memset");
-            ck(ar::nrc_train_step(c->net(), c->P, d, cnt, k * c->cfg.train_batch, c->cfg.train_batch, c->T,
-                                  c->cfg.learning_rate, ++c->step, c->scene->sm_count, nullptr, true,
-                                  c->tensor_path ? c->tc_err : nullptr), "cache training");
-            float l = 0.0f;
-            ck(cudaMemcpy(&l, c->T.loss, 4, cudaMemcpyDeviceToHost), "copy loss");
-            if (losses) losses[k] = l;
-        }
-    } catch (...) {
-        cudaFree(d); cudaFree(cnt);
-        throw;
+    NrcIo io(c, NrcIo::padded(n * sizeof(ar::NrcSample)) + 256);
+    ar::NrcSample* d = io.take<ar::NrcSample>(n);
+    int32_t* cnt = io.take<int32_t>(1);
+    const int32_t ni = static_cast<int32_t>(n);
+    if (n) ck(cudaMemcpy(d, samples, n * sizeof(ar::NrcSample), cudaMemcpyHostToDevice), "copy samples");
+    ck(cudaMemcpy(cnt, &ni, 4, cudaMemcpyHostToDevice), "copy count");
+    for (int k = 0; k < steps; ++k) {
+        ck(cudaMemset(c->T.loss, 0, 4), "memset");
+        ck(ar::nrc_train_step(c->net(), c->P, d, cnt, k * c->cfg.train_batch, c->cfg.train_batch, c->T,
+                              c->cfg.learning_rate, ++c->step, c->scene->sm_count, nullptr, true,
+                              c->tensor_path ? c->tc_err : nullptr), "cache training");
+        float l = 0.0f;
+        ck(cudaMemcpy(&l, c->T.loss, 4, cudaMemcpyDeviceToHost), "copy loss");
+        if (losses) losses[k] = l;
     }
-    cudaFree(d); cudaFree(cnt);
     return nrc_check(c, nullptr);
     AR_GUARD_END
 }
@@ -2015,10 +2114,21 @@ ar_status ar_spectral_rgb_lut(const float* tables, size_t count, int32_t res, in
         cudaGetLastError();
         return fail(AR_ERR_NO_DEVICE, "no CUDA device available");
     }
-    float* tab = dalloc<float>(count, "spectral tables");
-    float4* lam = dalloc<float4>(ar::kLambdaLutRes, "spectral lambda table");
-    int* err = dalloc<int>(1, "error word");
-    struct Free { void* a; void* b; void* c; ~Free() { cudaFree(a); cudaFree(b); cudaFree(c); } } fr{tab, lam, err};
+    // the library's static scratch of this device (cudaMalloc and cudaFree took
+    // a third of the call); a call that finds it in use allocates its own
+    static std::mutex scratch_lock;
+    std::unique_lock<std::mutex> held(scratch_lock, std::try_to_lock);
+    float* tab = nullptr;
+    float4* lam = nullptr;
+    int* err = nullptr;
+    struct Free { void* a = nullptr; void* b = nullptr; void* c = nullptr; ~Free() { cudaFree(a); cudaFree(b); cudaFree(c); } } fr;
+    if (held.owns_lock()) {
+        ck(ar::spectral_scratch(&tab, &lam, &err), "spectral scratch");
+    } else {
+        fr.a = tab = dalloc<float>(count, "spectral tables");
+        fr.b = lam = dalloc<float4>(ar::kLambdaLutRes, "spectral lambda table");
+        fr.c = err = dalloc<int>(1, "error word");
+    }
     ck(cudaMemcpy(tab, tables, count * sizeof(float), cudaMemcpyHostToDevice), "copy spectral tables");
     ck(cudaMemset(err, 0, sizeof(int)), "memset");
     cudaEvent_t e0, e1;

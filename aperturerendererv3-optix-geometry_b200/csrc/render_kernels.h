@@ -60,6 +60,8 @@ cudaError_t launch_material_basis(const MaterialRec* mats, int count, const floa
 // when a CTA's MMA wait runs out.
 cudaError_t launch_spectral_rgb_lut_tc(const float* tab, int res, float4* lut, int* err, int sm_count,
                                        cudaStream_t st);
+// The static scratch of ar_spectral_rgb_lut on the current device.
+cudaError_t spectral_scratch(float** tables, float4** lambda, int** err);
 cudaError_t launch_mean(const double* accum, int64_t n, double inv, float* out, cudaStream_t st);
 cudaError_t launch_add(const double* src, int64_t n, double* dst, cudaStream_t st);
 

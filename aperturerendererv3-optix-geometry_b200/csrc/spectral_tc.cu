@@ -220,6 +220,20 @@ __global__ void __launch_bounds__(2 * kLutRows) k_lut_rgb_tc(const float* __rest
 
 }  // namespace
 
+// Scratch of ar_spectral_rgb_lut, held by every device that loads the library:
+// its table block, the lambda table it does not return, an error word (86 KB).
+static __device__ __align__(256) float g_lut_tables[kTabFloats];
+static __device__ __align__(256) float4 g_lut_lambda[kLambdaLutRes];
+static __device__ int g_lut_error;
+
+cudaError_t spectral_scratch(float** tables, float4** lambda, int** err)
+{
+    cudaError_t e = cudaGetSymbolAddress(reinterpret_cast<void**>(tables), g_lut_tables);
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(reinterpret_cast<void**>(lambda), g_lut_lambda);
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(reinterpret_cast<void**>(err), g_lut_error);
+    return e;
+}
+
 cudaError_t launch_spectral_rgb_lut_tc(const float* tab, int res, float4* lut, int* err, int sm_count,
                                        cudaStream_t st)
 {
