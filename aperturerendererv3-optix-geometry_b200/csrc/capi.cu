@@ -98,10 +98,98 @@ private:
     bool changed_ = false;
 };
 
-constexpr int64_t kMaxPool = int64_t(1) << 21;  // paths in flight
+// Paths in flight (3.6 GB of path state).  Every iteration ends in the tails of
+// its traversal launches, ~0.1 ms of half-empty GPU whatever the pool holds, so
+// few long iterations beat many short ones, far past the L2 cache: the 64-sample
+// 1080p render of the 1M-triangle field takes 89.4 / 76.7 ms per 32 samples at
+// 2^20 / 2^21 paths, and per 64 samples 145.0 / 132.7 / 125.3 / 122.7 ms at
+// 2^21 / 2^22 / 2^23 / 2^24; 2^24 would take 7.2 GB for the last 2 %.
+constexpr int64_t kMaxPool = int64_t(1) << 23;
 // Paths left at which k_tail takes over from the wavefront: one path per lane
 // of its resident blocks.
 int tail_limit(int sm_count) { return ar::kTailBlocks * sm_count * ar::kTraceBlock; }
+
+// Path state of large renders: one block per device, lent to a render for its
+// duration, so scenes that render in turn share it.  A render that finds it lent
+// out allocates a block of its own; of the blocks that come back one is kept, the
+// larger, and it is freed with the device's last scene.  (A stream-ordered memory
+// pool did the same but took 25 ms longer to grow to 3.6 GB than cudaMalloc.)
+class PathMemory {
+public:
+    static void add_scene(int device)
+    {
+        std::lock_guard<std::mutex> g(lock());
+        ++entries()[device].scenes;
+    }
+    static void remove_scene(int device)
+    {
+        std::lock_guard<std::mutex> g(lock());
+        Entry& e = entries()[device];
+        if (--e.scenes > 0) return;
+        if (e.mem) cudaFree(e.mem);
+        e.mem = nullptr;
+        e.bytes = 0;
+    }
+    // at least `bytes` (set to the block's size) on the current device, or NULL
+    static char* take(int device, size_t& bytes)
+    {
+        {
+            std::lock_guard<std::mutex> g(lock());
+            Entry& e = entries()[device];
+            if (e.mem && e.bytes >= bytes) {
+                char* p = e.mem;
+                bytes = e.bytes;
+                e.mem = nullptr;
+                return p;
+            }
+            if (e.mem) cudaFree(e.mem);   // too small: its successor comes back instead
+            e.mem = nullptr;
+        }
+        void* p = nullptr;
+        if (cudaMalloc(&p, bytes) == cudaSuccess) return static_cast<char*>(p);
+        cudaGetLastError();
+        return nullptr;
+    }
+    static void give(int device, char* p, size_t bytes)   // idle: its last kernel has finished
+    {
+        std::lock_guard<std::mutex> g(lock());
+        Entry& e = entries()[device];
+        if (e.scenes > 0 && (!e.mem || e.bytes < bytes)) {
+            std::swap(p, e.mem);
+            e.bytes = bytes;
+        }
+        if (p) cudaFree(p);
+    }
+private:
+    struct Entry { char* mem = nullptr; size_t bytes = 0; int scenes = 0; };
+    static std::mutex& lock() { static std::mutex m; return m; }
+    static std::map<int, Entry>& entries() { static std::map<int, Entry> e; return e; }
+};
+
+// Lays the path state of `pool` paths out at b; returns its size (b may be NULL
+// to ask for it).
+size_t path_layout(ar::PathBuffers& B, char* b, int64_t pool)
+{
+    size_t off = 0;
+    auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
+    const size_t W = static_cast<size_t>(pool);
+    const size_t o_p0 = take(sizeof(ar::PathRec) * W), o_p1 = take(sizeof(ar::PathRec) * W);
+    const size_t o_hit = take(16 * W), o_qsh = take(4 * W * ar::kShadeBuckets);
+    const size_t o_sh = take(sizeof(ar::ShadowRec) * W), o_rt = take(sizeof(ar::RetireRec) * W);
+    const size_t o_ax0 = take(16 * W), o_ax1 = take(16 * W), o_sh3 = take(4 * W);
+    if (!b) return off;
+    B.pool[0] = reinterpret_cast<ar::PathRec*>(b + o_p0);
+    B.pool[1] = reinterpret_cast<ar::PathRec*>(b + o_p1);
+    B.hit = reinterpret_cast<int4*>(b + o_hit);
+    B.qsh = reinterpret_cast<int32_t*>(b + o_qsh);
+    B.shadow = reinterpret_cast<ar::ShadowRec*>(b + o_sh);
+    B.retire = reinterpret_cast<ar::RetireRec*>(b + o_rt);
+    B.aux[0] = reinterpret_cast<float4*>(b + o_ax0);
+    B.aux[1] = reinterpret_cast<float4*>(b + o_ax1);
+    B.shadow3 = reinterpret_cast<float*>(b + o_sh3);
+    B.capacity = static_cast<int32_t>(pool);
+    return off;
+}
 
 // What a batch needs besides its graph, kept by the scene of its first job from
 // one batch to the next: the jobs' workspaces as one allocation (at most
@@ -174,12 +262,12 @@ struct ar_scene {
     float bounds[6] = {0, 0, 0, 0, 0, 0};       // box of the BVH root (min xyz, max xyz)
     std::vector<ar::SdfRec> h_sdf;              // data pointers into h_volumes
     std::vector<ar::HostVolume> h_volumes;
-    // render workspace
+    // render workspace: per-pixel state, counters, traversal overflow
     char* ws = nullptr;
-    size_t ws_bytes = 0;
-    int64_t ws_wave = 0;
     int64_t ws_pix = 0;
-    ar::PathBuffers bufs{};
+    char* small_paths = nullptr;         // path state of small renders (PathState)
+    int64_t small_cap = 0;
+    bool counted = false;                // in PathMemory
     uint4* base0 = nullptr;
     uint2* base1 = nullptr;
     // the per-pixel generator states in base0/base1 are those of frame
@@ -207,46 +295,71 @@ struct ar_scene {
         if (ev1) cudaEventDestroy(ev1);
         for (cudaEvent_t e : timer_ext) cudaEventDestroy(e);
         for (cudaEvent_t e : timer_sh) cudaEventDestroy(e);
+        if (small_paths) cudaFree(small_paths);
+        if (counted) PathMemory::remove_scene(device);
     }
 };
 
 namespace {
 
-// Carve the two path pools, side arrays, queues and per-pixel buffers from one
-// allocation (re-used across calls; grown when a larger pool or image comes).
-void ensure_workspace(ar_scene* s, int64_t pool, int64_t npix)
+// The path state of one render: up to kSmallPool paths from the scene's own
+// memory (grown as needed), above that PathMemory's block.
+constexpr int64_t kSmallPool = int64_t(1) << 18;
+class PathState {
+public:
+    ar::PathBuffers B{};
+    // `pool` paths, or fewer when memory is short (down to kSmallPool)
+    PathState(ar_scene* s, int64_t pool, cudaStream_t st) : s_(s), st_(st)
+    {
+        while (pool > kSmallPool) {
+            bytes_ = path_layout(B, nullptr, pool);
+            mem_ = PathMemory::take(s->device, bytes_);
+            if (mem_) {
+                path_layout(B, mem_, pool);
+                return;
+            }
+            pool = std::max(kSmallPool, (pool + 1) / 2);
+        }
+        if (s->small_cap < pool) {
+            if (s->small_paths) cudaFree(s->small_paths);
+            s->small_paths = nullptr;
+            s->small_cap = 0;
+            s->small_paths = dalloc<char>(path_layout(B, nullptr, pool), "path state");
+            s->small_cap = pool;
+        }
+        path_layout(B, s->small_paths, pool);
+    }
+    ~PathState()
+    {
+        if (!mem_) return;
+        cudaStreamSynchronize(st_);   // done already, except after an error
+        PathMemory::give(s_->device, mem_, bytes_);
+    }
+    PathState(const PathState&) = delete;
+    PathState& operator=(const PathState&) = delete;
+private:
+    ar_scene* s_;
+    char* mem_ = nullptr;
+    size_t bytes_ = 0;
+    cudaStream_t st_;
+};
+
+// Carve the per-pixel buffers and counters from one allocation (re-used across
+// calls; grown when a larger image comes).
+void ensure_workspace(ar_scene* s, int64_t npix)
 {
-    if (s->ws && s->ws_wave >= pool && s->ws_pix >= npix) return;
+    if (s->ws && s->ws_pix >= npix) return;
     if (s->ws) { cudaFree(s->ws); s->ws = nullptr; }
-    pool = std::max(pool, s->ws_wave);
-    npix = std::max(npix, s->ws_pix);
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
-    const size_t W = static_cast<size_t>(pool), N = static_cast<size_t>(npix);
-    const size_t o_p0 = take(sizeof(ar::PathRec) * W), o_p1 = take(sizeof(ar::PathRec) * W);
-    const size_t o_hit = take(16 * W), o_qsh = take(4 * W * ar::kShadeBuckets);
-    const size_t o_sh = take(sizeof(ar::ShadowRec) * W), o_rt = take(sizeof(ar::RetireRec) * W);
-    const size_t o_ax0 = take(16 * W), o_ax1 = take(16 * W), o_sh3 = take(4 * W);
+    const size_t N = static_cast<size_t>(npix);
     const size_t o_b0 = take(16 * N), o_b1 = take(8 * N), o_acc = take(24 * N), o_fout = take(12 * N);
     const size_t o_cnt = take(sizeof(ar::PoolCtl)), o_stats = take(64), o_err = take(64);
     const size_t o_ovf = take(static_cast<size_t>(s->grid_trace) * ar::kTraceBlock * ar::kStackOverflow * 4);
     s->ws = dalloc<char>(off, "render workspace");
-    s->ws_bytes = off;
-    s->ws_wave = pool;
     s->ws_pix = npix;
     s->rng_valid = false;
     char* b = s->ws;
-    ar::PathBuffers& B = s->bufs;
-    B.pool[0] = reinterpret_cast<ar::PathRec*>(b + o_p0);
-    B.pool[1] = reinterpret_cast<ar::PathRec*>(b + o_p1);
-    B.hit = reinterpret_cast<int4*>(b + o_hit);
-    B.qsh = reinterpret_cast<int32_t*>(b + o_qsh);
-    B.shadow = reinterpret_cast<ar::ShadowRec*>(b + o_sh);
-    B.retire = reinterpret_cast<ar::RetireRec*>(b + o_rt);
-    B.aux[0] = reinterpret_cast<float4*>(b + o_ax0);
-    B.aux[1] = reinterpret_cast<float4*>(b + o_ax1);
-    B.shadow3 = reinterpret_cast<float*>(b + o_sh3);
-    B.capacity = static_cast<int32_t>(pool);
     s->base0 = reinterpret_cast<uint4*>(b + o_b0);
     s->base1 = reinterpret_cast<uint2*>(b + o_b1);
     s->accum = reinterpret_cast<double*>(b + o_acc);
@@ -379,9 +492,11 @@ ar_status run_render(ar_scene* s, const ar_camera* cam, const ar_render_params* 
         fp.guide = *guide;
     }
     if (dn) fp.dn = *dn;
-    ensure_workspace(s, pool, npix);
-    PathBuffers B = s->bufs;
-    B.capacity = static_cast<int32_t>(pool);
+    ensure_workspace(s, npix);
+    PathState state(s, pool, st);
+    const PathBuffers& B = state.B;
+    pool = B.capacity;
+    fp.pool = static_cast<int32_t>(pool);
     if (!s->ev0) { ck(cudaEventCreate(&s->ev0), "event"); ck(cudaEventCreate(&s->ev1), "event"); }
     ck(cudaEventRecord(s->ev0, st), "event record");
     // curand_init of every pixel (a skip-ahead per pixel) only when the stored
@@ -582,6 +697,8 @@ ar_status ar_scene_create_ex(const ar_object_desc* objects, size_t count, const 
     }
     cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, device);
     try {
+        PathMemory::add_scene(device);
+        s->counted = true;
         auto own = [&](void* p, size_t bytes) { s->owned.push_back(p); s->device_bytes += static_cast<int64_t>(bytes); return p; };
         ar::SceneView& v = s->view;
         v.nodes = static_cast<const ar::WideNode*>(own(upload(hs.nodes, "nodes"), hs.nodes.size() * sizeof(ar::WideNode)));
@@ -913,27 +1030,13 @@ struct JobWs {
 // Lays the workspace out at b; returns its size (b may be NULL to ask for it).
 size_t job_layout(JobWs& w, char* b, int64_t pool, int64_t npix, int grid_trace)
 {
-    size_t off = 0;
+    size_t off = path_layout(w.B, b, pool);
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
-    const size_t W = static_cast<size_t>(pool), N = static_cast<size_t>(npix);
-    const size_t o_p0 = take(sizeof(ar::PathRec) * W), o_p1 = take(sizeof(ar::PathRec) * W);
-    const size_t o_hit = take(16 * W), o_qsh = take(4 * W * ar::kShadeBuckets);
-    const size_t o_sh = take(sizeof(ar::ShadowRec) * W), o_rt = take(sizeof(ar::RetireRec) * W);
-    const size_t o_ax0 = take(16 * W), o_ax1 = take(16 * W), o_sh3 = take(4 * W);
+    const size_t N = static_cast<size_t>(npix);
     const size_t o_b0 = take(16 * N), o_b1 = take(8 * N), o_acc = take(24 * N);
     const size_t o_cnt = take(sizeof(ar::PoolCtl)), o_stats = take(64), o_err = take(64);
     const size_t o_ovf = take(static_cast<size_t>(grid_trace) * ar::kTraceBlock * ar::kStackOverflow * 4);
     if (!b) return off;
-    w.B.pool[0] = reinterpret_cast<ar::PathRec*>(b + o_p0);
-    w.B.pool[1] = reinterpret_cast<ar::PathRec*>(b + o_p1);
-    w.B.hit = reinterpret_cast<int4*>(b + o_hit);
-    w.B.qsh = reinterpret_cast<int32_t*>(b + o_qsh);
-    w.B.shadow = reinterpret_cast<ar::ShadowRec*>(b + o_sh);
-    w.B.retire = reinterpret_cast<ar::RetireRec*>(b + o_rt);
-    w.B.aux[0] = reinterpret_cast<float4*>(b + o_ax0);
-    w.B.aux[1] = reinterpret_cast<float4*>(b + o_ax1);
-    w.B.shadow3 = reinterpret_cast<float*>(b + o_sh3);
-    w.B.capacity = static_cast<int32_t>(pool);
     w.base0 = reinterpret_cast<uint4*>(b + o_b0);
     w.base1 = reinterpret_cast<uint2*>(b + o_b1);
     w.accum = reinterpret_cast<double*>(b + o_acc);
@@ -1095,7 +1198,7 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
     int64_t totalAll = 0;
     for (int j = 0; j < njobs; ++j)
         totalAll += static_cast<int64_t>(jobs[j].camera.width) * jobs[j].camera.height * jobs[j].params.spp;
-    const int64_t budget = path_budget > 0 ? path_budget : (int64_t(1) << 22);
+    const int64_t budget = path_budget > 0 ? path_budget : (int64_t(1) << 23);
     // Iterations per pass of the loop: as many as the fullest pool needs to start
     // all its samples, and some to bring the last paths under the tail's limit
     // (default; 16 whatever the batch made a graph of 1,900 nodes for 12 stills,
@@ -1301,7 +1404,7 @@ ar_status ar_trace_rays(ar_scene* s, const float* rays, size_t n, int32_t any_hi
     AR_GUARD_BEGIN
     DeviceGuard g(s->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (!s->err) ensure_workspace(s, 1, 1);
+    if (!s->err) ensure_workspace(s, 1);
     ck(cudaMemsetAsync(s->err, 0, 64, st), "memset err");
     const float4* drays;
     int32_t* dobj;

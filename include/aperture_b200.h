@@ -510,11 +510,12 @@ typedef struct ar_batch_stats {
  * the benchmark; the reference renders one camera at a time, scene.cu:276-306).
  * Every job keeps its own wavefront pool; the batch is ONE launch of a CUDA
  * graph whose WHILE conditional node repeats a body of iterations_per_graph
- * (0 = 16; rounded up to even) wavefront iterations of every job -- each job
+ * (0 = as many as the pools need to start all samples plus 3, at most 16;
+ * rounded up to even) wavefront iterations of every job -- each job
  * on its own branch so small jobs run side by side -- followed by a drain test
  * that sets the node's condition on the device until every job has retired
  * all of its paths (no host round trip between passes).  path_budget (0 =
- * 2^22) paths in flight are shared among the jobs by their share of the work
+ * 2^23) paths in flight are shared among the jobs by their share of the work
  * (a job's own params.wave_paths overrides).  All scenes on one device.
  * Outputs are written on `stream`; the call returns when they are complete. */
 ar_status ar_render_batch(const ar_job* jobs, int32_t njobs, int32_t iterations_per_graph, int64_t path_budget,
@@ -526,7 +527,7 @@ typedef struct ar_batch_tuning {
     int32_t candidates;            /* configurations timed                         */
     int64_t path_budget;           /* chosen in-flight path budget                 */
     float best_ms;                 /* probe time of the chosen configuration       */
-    float default_ms;              /* probe time of the defaults (16, 2^22)        */
+    float default_ms;              /* probe time of 16 iterations and 2^22 paths   */
     int32_t trace_blocks_per_sm;   /* chosen traversal grid per job (0: occupancy) */
     int32_t shade_blocks_per_sm;   /* chosen shading/generation/retirement grid    */
 } ar_batch_tuning;

@@ -73,3 +73,30 @@ def test_lookup_tables_in_two_threads():
     for _ in range(4):
         x, y = together(lambda: spectral_rgb_lut(24, LUT_TENSOR, ta)[0].cpu(), lambda: spectral_rgb_lut(40, LUT_TENSOR, tb)[0].cpu())
         assert bool((x == a).all()) and bool((y == b).all())
+
+
+@pytest.mark.gpu
+def test_scenes_share_the_path_state_of_large_renders(box_objects, small_spheres_objects):
+    """Renders above the size a scene keeps for itself: two scenes in turn, growing
+    and shrinking, and both at once from two threads."""
+    box, sph = Scene(box_objects), Scene(small_spheres_objects)
+    cam = scenes.spheres_camera(400, 300)
+    cam.position.z, cam.position.y = -45.0, 8.0
+    work = [(box, scenes.box_camera(300, 300), 4), (sph, cam, 3), (box, scenes.box_camera(700, 500), 2), (sph, cam, 9),
+            (box, scenes.box_camera(30, 20), 2)]
+
+    def image(w):
+        scene, c, spp = w
+        return scene.render(c, make_params(spp=spp, max_depth=5))[0]
+    ref = [image(w) for w in work]
+    for k in (3, 0, 4, 1, 2, 3):
+        np.testing.assert_allclose(image(work[k]), ref[k], rtol=1e-6, atol=1e-7)
+    for _ in range(3):
+        a, b = together(lambda: image(work[2]), lambda: image(work[3]))
+        np.testing.assert_allclose(a, ref[2], rtol=1e-6, atol=1e-7)
+        np.testing.assert_allclose(b, ref[3], rtol=1e-6, atol=1e-7)
+    box.close()   # the other scene still renders, and a new one after the last has gone
+    np.testing.assert_allclose(image(work[1]), ref[1], rtol=1e-6, atol=1e-7)
+    sph.close()
+    again = Scene(box_objects)
+    np.testing.assert_allclose(image((again,) + work[0][1:]), ref[0], rtol=1e-6, atol=1e-7)
