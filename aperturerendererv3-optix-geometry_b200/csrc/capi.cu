@@ -105,9 +105,12 @@ private:
 // 2^20 / 2^21 paths, and per 64 samples 145.0 / 132.7 / 125.3 / 122.7 ms at
 // 2^21 / 2^22 / 2^23 / 2^24; 2^24 would take 7.2 GB for the last 2 %.
 constexpr int64_t kMaxPool = int64_t(1) << 23;
-// Paths left at which k_tail takes over from the wavefront: one path per lane
-// of its resident blocks.
-int tail_limit(int sm_count) { return ar::kTailBlocks * sm_count * ar::kTraceBlock; }
+// Paths left at which k_tail takes over from the wavefront: four for each of its
+// lanes (151,552).  One-sample images of box / sphere scene, microseconds by the
+// tail kernel against the wavefront: 64,000 pixels 335 / 400 against 395 / 708,
+// 76,800 383 / 450 against 415 / 750, 120,000 572 / 526 against 508 / 792,
+// 147,456 594 / 628 against 506 / 779.
+int tail_limit(int sm_count) { return 4 * sm_count * ar::kTailBlock; }
 
 // Path state of large renders: one block per device, lent to a render for its
 // duration, so scenes that render in turn share it.  A render that finds it lent

@@ -12,7 +12,7 @@ namespace ar {
 constexpr int kTraceBlock = 128;  // threads per traversal block (4 warps)
 constexpr int kTraceMinBlocks = 8;  // resident blocks per SM the traversal kernels are built for (<= 64 registers)
 constexpr int kShadeBlock = 256;
-constexpr int kTailBlocks = 3;    // resident blocks per SM of the tail kernel
+constexpr int kTailBlock = 256;   // threads of the tail kernel's one block per SM
 
 // Upload INTERSECT_EPS(0..8) to the current device.
 cudaError_t set_intersect_eps(const float* tab9);

@@ -11,9 +11,10 @@
 //
 // Bound: instruction fetch and the latency of one path after the other (ncu on
 // the 160x120 preview, 19,200 paths: issue slots 17 % busy, half of a warp's wait
-// for instructions, 61 % of the fetches hit).  Few paths are spread over more
-// warps, 16 to 32 per warp: 240 us for that preview against 247 with 32 and 272
-// with 11 to a warp and warps that run free.
+// for instructions, 61 % of the fetches hit).  So one block of 8 warps per SM,
+// whose warps advance segment by segment together, and few paths spread over all
+// warps, 16 to 32 each.  That preview: 272 us with three blocks of 4 warps that
+// run free, 240 with the warps of a block together, 206 with one block.
 #include "path_stages.cuh"
 
 #include <algorithm>
@@ -22,7 +23,7 @@ namespace ar {
 
 namespace {
 
-constexpr size_t kTailSmem = static_cast<size_t>(kStackShared) * kTraceBlock * 4;
+constexpr size_t kTailSmem = static_cast<size_t>(kStackShared) * kTailBlock * 4;
 
 template <bool kAny>
 __device__ __forceinline__ void traverse_one(const SceneView& s, RayState& r, uint32_t* stack, uint32_t* ovf, int* err)
@@ -33,7 +34,7 @@ __device__ __forceinline__ void traverse_one(const SceneView& s, RayState& r, ui
 }
 
 template <bool kExt, int kSpec, bool kNrc, bool kGuide>
-__global__ void __launch_bounds__(kTraceBlock, kSpec == 4 ? 2 : kTailBlocks)
+__global__ void __launch_bounds__(kTailBlock, 1)
 k_tail(SceneView s, FrameParams fp, PathBuffers B, int cur, PoolCtl* ctl, unsigned long long* stats, uint32_t* ovf_base,
        int* err, double* accum, ar_path_record* rec, int limit)
 {
@@ -44,7 +45,7 @@ k_tail(SceneView s, FrameParams fp, PathBuffers B, int cur, PoolCtl* ctl, unsign
     uint32_t* stack = lane_stack(smem);
     uint32_t* ovf = thread_overflow(ovf_base);
     const PathRec* pool = pool_of(B, cur);
-    const int warps = gridDim.x * (kTraceBlock / 32);
+    const int warps = gridDim.x * (kTailBlock / 32);
     const int lanes = min(32, max(16, (n + warps - 1) / warps));   // paths per warp
     // warps of consecutive index on different SMs
     const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
@@ -132,9 +133,9 @@ cudaError_t launch_tail(const SceneView& s, const FrameParams& fp, const PathBuf
                         int limit, int sm_count, cudaStream_t st)
 {
     const bool ext = s.num_sdf > 0 || s.has_medium;
-    const int grid = kTailBlocks * sm_count;
+    const int grid = sm_count;
     auto go = [&](auto kernel) {
-        kernel<<<grid, kTraceBlock, kTailSmem, st>>>(s, fp, B, cur, ctl, stats, ovf, err, accum, rec, limit);
+        kernel<<<grid, kTailBlock, kTailSmem, st>>>(s, fp, B, cur, ctl, stats, ovf, err, accum, rec, limit);
     };
     if (fp.spectral == 4 && fp.nrc.enabled) ext ? go(k_tail<true, 4, true, false>) : go(k_tail<false, 4, true, false>);
     else if (fp.spectral == 4) ext ? go(k_tail<true, 4, false, false>) : go(k_tail<false, 4, false, false>);

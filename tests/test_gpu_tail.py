@@ -8,7 +8,7 @@ import pytest
 import scenes
 from aperture_b200 import Scene, make_params
 
-BLOCKS, BLOCK = 3, 128   # resident blocks per SM and threads per block of the kernel
+LANES, PER_LANE = 256, 4   # lanes per SM of the kernel, and paths per lane up to which it is used
 
 
 def tables(seed=3):
@@ -59,7 +59,7 @@ def test_tail_traces_the_wavefronts_paths(kind, spectral, nee):
 def test_path_counts_around_the_limit(total):
     scene, camera = scene_of("box")
     sms = __import__("torch").cuda.get_device_properties(0).multi_processor_count
-    limit = BLOCKS * sms * BLOCK
+    limit = LANES * PER_LANE * sms
     n = {"limit": limit, "limit+1": limit + 1}.get(total, total)
     cam = camera(n, 1)
     one = scene.debug_paths(cam, make_params(spp=1, max_depth=6))
