@@ -43,8 +43,12 @@ constexpr int kLutWLayer = kLutN * kLutK * 2;                 // bytes of one bf
 constexpr int kLutWOut = kLutNOut * kLutK * 2;
 constexpr int kLutWBytes = 3 * ((kLutLayers - 1) * kLutWLayer + kLutWOut);   // three splits
 constexpr int kLutABytes = kLutRows * kLutK * 2;              // one bf16 split of the activations
-constexpr int kLutSmem = kLutWBytes + 6 * kLutABytes + 64;   // weights, two tiles' A operands, barriers
-constexpr int kLutCols = 32;                                  // TMEM columns (fp32 accumulators)
+constexpr int kLutTiles = 6;                                  // tiles side by side in a CTA
+constexpr int kLutBarriers = kLutWBytes + kLutTiles * 3 * kLutABytes;   // offset of the mbarriers
+constexpr int kLutBias = kLutBarriers + 128;                 // offset of the hidden layers' biases (fp32)
+constexpr int kLutSmem = kLutBias + (kLutLayers - 1) * kLutN * 4;   // weights, the tiles' A operands, barriers, biases
+constexpr int kLutCols = 32;                                  // TMEM columns of a tile (fp32 accumulators)
+constexpr int kLutAllocCols = kLutTiles * kLutCols <= 128 ? 128 : 256;   // a power of two
 constexpr uint32_t kLutSpinLimit = 1u << 22;
 
 // byte offset of split j of layer l's weights
@@ -61,16 +65,32 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16* t)
     t[2] = __float2bfloat16_rn(r1 - __bfloat162float(t[1]));
 }
 
+// The three bf16 terms of two values at once, as packed pairs (a in the low
+// half).  The packed conversion does not go through the conversion unit that the
+// scalar one occupies (56 % busy, the kernel's busiest pipe).
+__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b)
+{
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ void split3_pair(float a, float b, uint32_t* t)
+{
+    t[0] = pack_bf16x2(a, b);
+    const float a1 = a - __uint_as_float(t[0] << 16), b1 = b - __uint_as_float(t[0] & 0xFFFF0000u);
+    t[1] = pack_bf16x2(a1, b1);
+    t[2] = pack_bf16x2(a1 - __uint_as_float(t[1] << 16), b1 - __uint_as_float(t[1] & 0xFFFF0000u));
+}
+
 // row t's 32 fp32 values as the three bf16 splits of the A operand
 __device__ __forceinline__ void store_row(unsigned char* sA, int t, const float* h)
 {
 #pragma unroll
     for (int kc = 0; kc < kLutK / 8; ++kc) {
-        __nv_bfloat16 v[3][8];
+        uint32_t v[3][4];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            __nv_bfloat16 s3[3];
-            split3(h[8 * kc + e], s3);
+        for (int e = 0; e < 4; ++e) {
+            uint32_t s3[3];
+            split3_pair(h[8 * kc + 2 * e], h[8 * kc + 2 * e + 1], s3);
             v[0][e] = s3[0];
             v[1][e] = s3[1];
             v[2][e] = s3[2];
@@ -78,7 +98,7 @@ __device__ __forceinline__ void store_row(unsigned char* sA, int t, const float*
 #pragma unroll
         for (int j = 0; j < 3; ++j)
             *reinterpret_cast<uint4*>(sA + j * kLutABytes + tc_chunk_offset(kLutRows, t, kc)) =
-                *reinterpret_cast<const uint4*>(v[j]);
+                make_uint4(v[j][0], v[j][1], v[j][2], v[j][3]);
     }
 }
 
@@ -90,7 +110,7 @@ namespace {
 // A operand, mbarrier and 32 tensor-memory columns and synchronises on a named
 // barrier of its own, so one half's epilogue (tcgen05.ld, bias, ReLU, split,
 // store) overlaps the other half's MMAs.  The weights are shared.
-__global__ void __launch_bounds__(2 * kLutRows) k_lut_rgb_tc(const float* __restrict__ tab, int res,
+__global__ void __launch_bounds__(kLutTiles * kLutRows, 1) k_lut_rgb_tc(const float* __restrict__ tab, int res,
                                                              float4* __restrict__ lut, int* err)
 {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -99,11 +119,11 @@ __global__ void __launch_bounds__(2 * kLutRows) k_lut_rgb_tc(const float* __rest
     const int t = threadIdx.x & (kLutRows - 1);        // row within the tile
     const int warp = threadIdx.x >> 5;
     unsigned char* sA = smem + kLutWBytes + half * 3 * kLutABytes;
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + kLutWBytes + 6 * kLutABytes) + half;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kLutWBytes + 6 * kLutABytes + 16);
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + kLutBarriers) + half;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kLutBarriers + 64);
 
     // weights [out][in] of every layer as three bf16 splits, B operands (N rows x K)
-    for (int e = threadIdx.x; e < kLutLayers * kLutN * kLutK; e += 2 * kLutRows) {
+    for (int e = threadIdx.x; e < kLutLayers * kLutN * kLutK; e += kLutTiles * kLutRows) {
         const int l = e / (kLutN * kLutK), rem = e - l * (kLutN * kLutK);
         const int n = rem / kLutK, k = rem - n * kLutK;
         const int R = l == kLutLayers - 1 ? kLutNOut : kLutN;
@@ -118,13 +138,16 @@ __global__ void __launch_bounds__(2 * kLutRows) k_lut_rgb_tc(const float* __rest
             *reinterpret_cast<__nv_bfloat16*>(sW + lut_w_offset(l, j) + tc_chunk_offset(R, n, k / 8) + (k % 8) * 2) =
                 s3[j];
     }
+    float* sBias = reinterpret_cast<float*>(smem + kLutBias);
+    for (int e = threadIdx.x; e < (kLutLayers - 1) * kLutN; e += kLutTiles * kLutRows)
+        sBias[e] = e < kLutN ? tab[kTabRgbInB + e] : tab[kTabRgbBlkB + e - kLutN];
     if (t == 0) {   // thread 0 of each half: its mbarrier
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" : : "r"(smem_addr(mbar)), "r"(1) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     : : "r"(smem_addr(tmem_slot)), "r"(2 * kLutCols) : "memory");
+                     : : "r"(smem_addr(tmem_slot)), "r"(kLutAllocCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -137,8 +160,8 @@ __global__ void __launch_bounds__(2 * kLutRows) k_lut_rgb_tc(const float* __rest
     bool failed = false;
     const int64_t total = static_cast<int64_t>(res) * res * res;
     const float invRes = 1.0f / static_cast<float>(res);
-    for (int64_t tile = 2 * static_cast<int64_t>(blockIdx.x) + half; tile * kLutRows < total && !failed;
-         tile += 2 * static_cast<int64_t>(gridDim.x)) {
+    for (int64_t tile = kLutTiles * static_cast<int64_t>(blockIdx.x) + half; tile * kLutRows < total && !failed;
+         tile += kLutTiles * static_cast<int64_t>(gridDim.x)) {
         const int64_t vx = tile * kLutRows + t;
         const bool valid = vx < total;
         const int64_t v = valid ? vx : total - 1;
@@ -189,18 +212,29 @@ __global__ void __launch_bounds__(2 * kLutRows) k_lut_rgb_tc(const float* __rest
             failed = half_sync_or(half, late);   // the same decision in every thread of the half
             if (failed) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t acc[kLutN];
-            tc_ld32(taddr, acc);
-            if (l == 0) {
+            // the accumulators in two halves of 16: registers for 6 tiles
 #pragma unroll
-                for (int i = 0; i < kLutN; ++i) h[i] = fmaxf(__uint_as_float(acc[i]) + __ldg(tab + kTabRgbInB + i), 0.0f);
-            } else if (l < kLutLayers - 1) {
-                const float* B = tab + kTabRgbBlkB + (l - 1) * 32;
+            for (int c = 0; c < 2; ++c) {
+                if (c == 1 && l == kLutLayers - 1) break;
+                uint32_t acc[16];
+                tc_ld16(taddr + 16 * c, acc);
+                if (l < kLutLayers - 1) {
+                    const float4* B = reinterpret_cast<const float4*>(sBias + l * kLutN + 16 * c);
 #pragma unroll
-                for (int i = 0; i < kLutN; ++i) h[i] = h[i] + fmaxf(__uint_as_float(acc[i]) + __ldg(B + i), 0.0f);
-            } else {
+                    for (int q = 0; q < 4; ++q) {
+                        const float4 b = B[q];
+                        const float z[4] = {__uint_as_float(acc[4 * q]) + b.x, __uint_as_float(acc[4 * q + 1]) + b.y,
+                                            __uint_as_float(acc[4 * q + 2]) + b.z, __uint_as_float(acc[4 * q + 3]) + b.w};
 #pragma unroll
-                for (int i = 0; i < kSpecKernel; ++i) out[i] = __uint_as_float(acc[i]) * scale;
+                        for (int e = 0; e < 4; ++e) {
+                            const int i = 16 * c + 4 * q + e;
+                            h[i] = (l == 0 ? 0.0f : h[i]) + fmaxf(z[e], 0.0f);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < kSpecKernel; ++i) out[i] = __uint_as_float(acc[i]) * scale;
+                }
             }
         }
         if (failed) break;
@@ -215,7 +249,7 @@ __global__ void __launch_bounds__(2 * kLutRows) k_lut_rgb_tc(const float* __rest
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" : : "r"(*tmem_slot), "r"(2 * kLutCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" : : "r"(*tmem_slot), "r"(kLutAllocCols) : "memory");
 }
 
 }  // namespace
@@ -241,8 +275,8 @@ cudaError_t launch_spectral_rgb_lut_tc(const float* tab, int res, float4* lut, i
     if (e != cudaSuccess) return e;
     const int64_t total = static_cast<int64_t>(res) * res * res;
     const int64_t tiles = (total + kLutRows - 1) / kLutRows;
-    const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((tiles + 1) / 2, int64_t(sm_count) * 2)));
-    k_lut_rgb_tc<<<grid, 2 * kLutRows, kLutSmem, st>>>(tab, res, lut, err);
+    const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((tiles + kLutTiles - 1) / kLutTiles, sm_count)));
+    k_lut_rgb_tc<<<grid, kLutTiles * kLutRows, kLutSmem, st>>>(tab, res, lut, err);
     return cudaGetLastError();
 }
 
