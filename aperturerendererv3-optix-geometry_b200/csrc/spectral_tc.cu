@@ -7,16 +7,27 @@
 //
 // A tile is 128 voxels, one per thread; every layer is one 128 x 32 x 32
 // matrix product on tcgen05.mma (kind::f16) with fp32 accumulators in tensor
-// memory.  A CTA of 256 threads runs two tiles side by side.  The MMA takes bf16 operands, so fp32 accuracy comes from splitting
+// memory.  The MMA takes bf16 operands, so fp32 accuracy comes from splitting
 // both operands into three bf16 terms, x = x0 + x1 + x2 (x0 = bf16(x),
-// x1 = bf16(x - x0), x2 = bf16(x - x0 - x1): 24 significant bits), and
-// accumulating the six products whose order is at most 2 (x2 w0, x1 w1,
-// x0 w2, x1 w0, x0 w1, x0 w0, smallest first).  The activations stay fp32 in
-// the registers of the row's thread between layers (bias, ReLU, residual sum
-// from tcgen05.ld); only the next layer's split operand goes back to shared
-// memory.  Entries differ from the SIMT build (one thread per voxel, fmaf in
-// input order) by the summation order and the dropped products of order 3
-// and above: a few fp32 ulps, measured by ar_spectral_rgb_lut.
+// x1 = bf16(x - x0), x2 = bf16(x - x0 - x1): 24 significant bits), and adding the
+// six products whose order is at most 2: x0 w0; x1 w0, x0 w1; x2 w0, x1 w1,
+// x0 w2.  The weight splits lie one below the other in one operand, so each
+// activation split is one product with as many of them as it needs, and the
+// products of one order meet in one of three accumulators; the epilogue adds
+// these, smallest first.  The activations stay fp32 in the registers of the row's
+// thread between layers (bias, ReLU, residual sum from tcgen05.ld); only the next
+// layer's split operand goes back to shared memory.  Entries differ from the SIMT
+// build (one thread per voxel, fmaf in input order) by the summation order and
+// the dropped products of order 3 and above: a few fp32 ulps, measured by
+// ar_spectral_rgb_lut.
+//
+// A CTA of 640 threads runs five tiles side by side, one CTA per SM (registers,
+// and 480 of the 512 tensor-memory columns).  Bound: the latency of a layer's
+// chain (operand to shared memory, MMA, commit, accumulator back) and the issue
+// slots of its fp32 part.  160^3 table: 1212 us with two tiles per CTA and two
+// CTAs per SM, twelve 32-column MMAs per layer and scalar conversions; 1063 us
+// with six tiles in one CTA; 960 us with packed conversions; 840 us with
+// six MMAs per layer and five tiles.
 //
 // Every wait is bounded; a CTA whose MMA does not complete within the limit
 // sets the error word, waits once more for its commit, frees its tensor
@@ -37,25 +48,23 @@ namespace {
 constexpr int kLutRows = 128;                                 // voxels per CTA tile (M)
 constexpr int kLutLayers = 2 + kSpecBlocks;                   // input, 7 blocks, output
 constexpr int kLutN = 32;                                     // width of the hidden layers
-constexpr int kLutNOut = 16;                                  // output layer N (4 used)
+constexpr int kLutNOut = 32;                                  // output layer N (4 used, the others' weights are 0)
 constexpr int kLutK = 32;
 constexpr int kLutWLayer = kLutN * kLutK * 2;                 // bytes of one bf16 weight split (hidden)
 constexpr int kLutWOut = kLutNOut * kLutK * 2;
 constexpr int kLutWBytes = 3 * ((kLutLayers - 1) * kLutWLayer + kLutWOut);   // three splits
 constexpr int kLutABytes = kLutRows * kLutK * 2;              // one bf16 split of the activations
-constexpr int kLutTiles = 6;                                  // tiles side by side in a CTA
+constexpr int kLutTiles = 5;                                  // tiles side by side in a CTA
 constexpr int kLutBarriers = kLutWBytes + kLutTiles * 3 * kLutABytes;   // offset of the mbarriers
 constexpr int kLutBias = kLutBarriers + 128;                 // offset of the hidden layers' biases (fp32)
 constexpr int kLutSmem = kLutBias + (kLutLayers - 1) * kLutN * 4;   // weights, the tiles' A operands, barriers, biases
-constexpr int kLutCols = 32;                                  // TMEM columns of a tile (fp32 accumulators)
-constexpr int kLutAllocCols = kLutTiles * kLutCols <= 128 ? 128 : 256;   // a power of two
+constexpr int kLutCols = 3 * kLutN;                          // TMEM columns of a tile (three fp32 accumulators)
+constexpr int kLutAllocCols = 512;
 constexpr uint32_t kLutSpinLimit = 1u << 22;
 
-// byte offset of split j of layer l's weights
-__host__ __device__ constexpr int lut_w_offset(int l, int j)
-{
-    return j * ((kLutLayers - 1) * kLutWLayer + kLutWOut) + l * kLutWLayer;
-}
+// byte offset of layer l's weights: the three splits' rows one after the other, a
+// B operand of 3 N rows
+__host__ __device__ constexpr int lut_w_offset(int l) { return 3 * l * kLutWLayer; }
 
 __device__ __forceinline__ void split3(float x, __nv_bfloat16* t)
 {
@@ -106,16 +115,16 @@ __device__ __forceinline__ void store_row(unsigned char* sA, int t, const float*
 
 namespace {
 
-// Two halves of 128 threads run two tiles side by side: each half has its own
-// A operand, mbarrier and 32 tensor-memory columns and synchronises on a named
-// barrier of its own, so one half's epilogue (tcgen05.ld, bias, ReLU, split,
-// store) overlaps the other half's MMAs.  The weights are shared.
+// Groups of 128 threads run the tiles side by side: each group has its own A
+// operand, mbarrier and 96 tensor-memory columns and synchronises on a named
+// barrier of its own, so one group's epilogue (tcgen05.ld, bias, ReLU, split,
+// store) overlaps the others' MMAs.  The weights are shared.
 __global__ void __launch_bounds__(kLutTiles * kLutRows, 1) k_lut_rgb_tc(const float* __restrict__ tab, int res,
                                                              float4* __restrict__ lut, int* err)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char* sW = smem;
-    const int half = threadIdx.x >> 7;                 // which tile of the pair
+    const int half = threadIdx.x >> 7;                 // which tile of the CTA
     const int t = threadIdx.x & (kLutRows - 1);        // row within the tile
     const int warp = threadIdx.x >> 5;
     unsigned char* sA = smem + kLutWBytes + half * 3 * kLutABytes;
@@ -135,13 +144,13 @@ __global__ void __launch_bounds__(kLutTiles * kLutRows, 1) k_lut_rgb_tc(const fl
         __nv_bfloat16 s3[3];
         split3(w, s3);
         for (int j = 0; j < 3; ++j)
-            *reinterpret_cast<__nv_bfloat16*>(sW + lut_w_offset(l, j) + tc_chunk_offset(R, n, k / 8) + (k % 8) * 2) =
+            *reinterpret_cast<__nv_bfloat16*>(sW + lut_w_offset(l) + tc_chunk_offset(3 * R, j * R + n, k / 8) + (k % 8) * 2) =
                 s3[j];
     }
     float* sBias = reinterpret_cast<float*>(smem + kLutBias);
     for (int e = threadIdx.x; e < (kLutLayers - 1) * kLutN; e += kLutTiles * kLutRows)
         sBias[e] = e < kLutN ? tab[kTabRgbInB + e] : tab[kTabRgbBlkB + e - kLutN];
-    if (t == 0) {   // thread 0 of each half: its mbarrier
+    if (t == 0) {   // thread 0 of each group: its mbarrier
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" : : "r"(smem_addr(mbar)), "r"(1) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -153,7 +162,7 @@ __global__ void __launch_bounds__(kLutTiles * kLutRows, 1) k_lut_rgb_tc(const fl
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot + static_cast<uint32_t>(half * kLutCols);   // this half's columns
+    const uint32_t tmem = *tmem_slot + static_cast<uint32_t>(half * kLutCols);   // this group's columns
     const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);  // lanes of this warp's rows
     const uint32_t aBase = smem_addr(sA), wBase = smem_addr(sW), mb = smem_addr(mbar);
     uint32_t phase = 0;
@@ -189,17 +198,18 @@ __global__ void __launch_bounds__(kLutTiles * kLutRows, 1) k_lut_rgb_tc(const fl
             half_sync(half);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (t == 0) {
-                const uint32_t idesc = tc_idesc(kLutRows, N);
-                const int pa[6] = {2, 1, 0, 1, 0, 0}, pw[6] = {0, 1, 2, 0, 1, 0};   // smallest products first
+                // activation split p times the weight splits 0 .. 2 - p, as one product
+                // of (3 - p) N columns whose accumulators start at p N: accumulator o
+                // collects the products of order o
 #pragma unroll
-                for (int ks = 0; ks < kLutK / 16; ++ks)
+                for (int p = 0; p < 3; ++p)
 #pragma unroll
-                    for (int p = 0; p < 6; ++p) {
-                        const uint64_t da = tc_desc(aBase + static_cast<uint32_t>(pa[p] * kLutABytes + 2 * ks * kLutRows * 16),
+                    for (int ks = 0; ks < kLutK / 16; ++ks) {
+                        const uint64_t da = tc_desc(aBase + static_cast<uint32_t>(p * kLutABytes + 2 * ks * kLutRows * 16),
                                                     kLutRows * 16, 128);
-                        const uint64_t db = tc_desc(wBase + static_cast<uint32_t>(lut_w_offset(l, pw[p]) + 2 * ks * N * 16),
-                                                    static_cast<uint32_t>(N * 16), 128);
-                        tc_mma(tmem, da, db, idesc, (ks > 0 || p > 0) ? 1u : 0u);
+                        const uint64_t db = tc_desc(wBase + static_cast<uint32_t>(lut_w_offset(l) + 2 * ks * 3 * N * 16),
+                                                    static_cast<uint32_t>(3 * N * 16), 128);
+                        tc_mma(tmem + static_cast<uint32_t>(p * N), da, db, tc_idesc(kLutRows, (3 - p) * N), (ks > 0 || p > 0) ? 1u : 0u);
                     }
                 tc_commit(mb);
             }
@@ -209,15 +219,18 @@ __global__ void __launch_bounds__(kLutTiles * kLutRows, 1) k_lut_rgb_tc(const fl
                 if (++spins >= kLutSpinLimit) { late = true; break; }
             }
             phase ^= 1u;
-            failed = half_sync_or(half, late);   // the same decision in every thread of the half
+            failed = half_sync_or(half, late);   // the same decision in every thread of the group
             if (failed) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // the accumulators in two halves of 16: registers for 6 tiles
+            // the accumulators in two halves of 16: registers for all tiles
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 if (c == 1 && l == kLutLayers - 1) break;
-                uint32_t acc[16];
-                tc_ld16(taddr + 16 * c, acc);
+                uint32_t acc[16], acc1[16], acc2[16];
+                tc_ld16x3(taddr + 16 * c, static_cast<uint32_t>(N), acc, acc1, acc2);
+#pragma unroll
+                for (int i = 0; i < 16; ++i)   // smallest first
+                    acc[i] = __float_as_uint((__uint_as_float(acc2[i]) + __uint_as_float(acc1[i])) + __uint_as_float(acc[i]));
                 if (l < kLutLayers - 1) {
                     const float4* B = reinterpret_cast<const float4*>(sBias + l * kLutN + 16 * c);
 #pragma unroll
