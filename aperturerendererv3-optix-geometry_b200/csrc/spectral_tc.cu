@@ -26,7 +26,7 @@
 // chain (operand to shared memory, MMA, commit, accumulator back) and the issue
 // slots of its fp32 part.  160^3 table: 1212 us with two tiles per CTA and two
 // CTAs per SM, twelve 32-column MMAs per layer and scalar conversions; 1063 us
-// with six tiles in one CTA; 960 us with packed conversions; 840 us with
+// with six tiles in one CTA; 960 us with packed conversions; 850 us with
 // six MMAs per layer and five tiles.
 //
 // Every wait is bounded; a CTA whose MMA does not complete within the limit
