@@ -529,15 +529,15 @@ __device__ __forceinline__ bool ray_step(const SceneView& s, RayState& r, uint32
 
 // Persistent traversal loop shared by every ray-query kernel.  Each warp keeps
 // 32 rays in flight.  Lanes whose rays finish are refilled in batches of at
-// least refill_min(kAny) (or when the whole warp is idle): the refill stores
+// least kRefillMin (or when the whole warp is idle): the refill stores
 // their results and loads new queue entries (one atomic per warp per refill),
 // so the lane-divergent store/load code runs once for several lanes instead of
 // once per finishing lane, while no lane idles for long.  Measured on the
-// 1M-triangle sphere field: 8 for closest-hit queries; 16 for any-hit queries,
-// whose short lives make refills frequent (2 and 4 were 6-14 % slower for
-// both).  IO supplies load() -> item id or -1 when the entry finished without
-// traversal, and store().
-constexpr int refill_min(bool any) { return any ? 16 : 8; }
+// 1M-triangle sphere field (64 samples at 1080p, 2^23 paths in flight): closest
+// hits at thresholds 6 / 8 / 12 / 14 / 16 take 57.4 / 55.7 / 54.4 / 54.6 / 55.4 ms,
+// any hits at 8 / 12 / 16 / 20 take 31.0 / 30.6 / 30.9 / 31.7 ms.  IO supplies
+// load() -> item id or -1 when the entry finished without traversal, and store().
+constexpr int kRefillMin = 12;
 
 template <bool kAny, class IO, bool kCount = false>
 __device__ __forceinline__ void traverse_queue(const SceneView& s, IO& io, int n, int* fetch, uint32_t* stack,
@@ -551,7 +551,7 @@ __device__ __forceinline__ void traverse_queue(const SceneView& s, IO& io, int n
     bool exhausted = false;
     for (;;) {
         const unsigned idle = __ballot_sync(0xFFFFFFFFu, item < 0);
-        const bool refill = !exhausted && idle != 0u && (__popc(idle) >= refill_min(kAny) || idle == 0xFFFFFFFFu);
+        const bool refill = !exhausted && idle != 0u && (__popc(idle) >= kRefillMin || idle == 0xFFFFFFFFu);
         if ((refill || exhausted) && pend >= 0) {
             io.store(s, pend, r);
             if (kCount) {
