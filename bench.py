@@ -738,7 +738,10 @@ def run_ours(args) -> None:
             line["relmse_oracle"] = (f"FP64 per-pixel mean of 4096 spp of the same tracer (sample streams disjoint "
                                      f"from the timed renders', {ref_s:.1f} s); relMSE of one timed step's 64-spp image")
             del ref_img
-        if world == 1 and args.nrc != "off":
+        import spectral_tables
+        if world == 1 and args.nrc == "config3" and not spectral_tables.available():
+            line["nrc"] = {"unavailable": "spectral tables absent: the four-wavelength cache has no table to read"}
+        elif world == 1 and args.nrc != "off":
             line["nrc"] = measure_nrc(torch, dev, scene, args.nrc, stream, args.nrc_spp, args.nrc_c, args.nrc_steps)
         if world == 1 and args.configs > 0:
             line["other_configs"] = measure_configs(torch, dev, stream, args.configs)
