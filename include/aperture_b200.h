@@ -168,7 +168,9 @@ typedef struct ar_scene_info {
 
 /* Counters of one ar_render call.  Passing a stats pointer also times every
  * closest-hit and any-hit traversal launch with CUDA events on the caller's
- * stream (a few microseconds of overhead per launch). */
+ * stream (a few microseconds of overhead per launch).  The last paths of a
+ * render, and all of a small one, are traced by a kernel that does every stage:
+ * their queries are counted, its time is in total_ms only. */
 typedef struct ar_render_stats {
     int64_t paths;           /* camera paths traced                                  */
     int64_t extension_rays;  /* closest-hit BVH queries                              */
