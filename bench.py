@@ -51,7 +51,7 @@ WORKLOAD = ("config2: 800 icospheres x 1280 triangles + 2-triangle ground (1,024
 def config_block(n_gpus: int) -> dict:
     return {"workload": WORKLOAD, "triangles": 1024002, "width": WIDTH, "height": HEIGHT, "spp": SPP,
             "max_depth": DEPTH, "camera": "spheres_camera(): pos (0,30,-150), fov 60",
-            "l2": "flushed between timed steps (256 MiB write); path state 470 MB > L2",
+            "l2": "flushed between timed steps (256 MiB write); path state 3.6 GB > L2",
             "parallelism": f"replicas x{n_gpus}, FP64 accumulators reduced with NCCL" if n_gpus > 1 else "single GPU"}
 
 
@@ -512,7 +512,8 @@ def measure_config5(torch, dev, stream, njobs: int = 64) -> dict:
              for sp in specs]
     total_ms = st.total_ms + cache_ms
     return {"workload": f"{njobs} seeded jobs: config-2 generator with 10K-2M triangles (log-uniform), resolutions "
-                        "log-uniform 128-1024 per axis, spp in {4,16,64,256}, every second job four wavelengths, "
+                        "log-uniform 128-1024 per axis, spp in {4,16,64,256}, "
+                        + ("every second job four wavelengths, " if spectral_ok else "all RGB (spectral tables absent), ") +
                         "half the jobs with their own radiance cache (frames of up to 16 spp, trained online); jobs "
                         "without a cache in one launch of the batch graph (device-side loop), autotuned",
             "jobs": njobs, "ms": round(total_ms, 3),
