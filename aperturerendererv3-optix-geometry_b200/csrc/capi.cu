@@ -406,7 +406,7 @@ ar_status check_camera(const ar_camera* c)
 {
     if (!c) return fail(AR_ERR_INVALID_ARGUMENT, "camera is NULL");
     if (c->width <= 0 || c->height <= 0) return fail(AR_ERR_INVALID_ARGUMENT, "camera width/height must be positive");
-    if (static_cast<int64_t>(c->width) * c->height > (int64_t(1) << 28))
+    if (static_cast<int64_t>(c->width) * c->height > ar::kMaxImagePixels)
         return fail(AR_ERR_INVALID_ARGUMENT, "image larger than 2^28 pixels");
     if (!(c->fov_y_deg > 0.0f && c->fov_y_deg < 180.0f)) return fail(AR_ERR_INVALID_ARGUMENT, "fov_y_deg must be in (0, 180)");
     return AR_OK;

@@ -88,9 +88,12 @@ inline std::vector<uint32_t> xorwow_jump_table_pow2(int p) { return xorwow_jump_
 // Jumps of the per-pixel initialisation (k_rng_init), in units of one curand
 // subsequence (2^67 draws): 1 (the next pixel of a row of 8), 8 and 16 (rows of
 // an 8x4 pixel block), 32, 64 and 128 (blocks of a group of 8), then 256 2^k for
-// the bits of the group index (images have at most 2^28 pixels); before them the
-// frame bits, 2^32 2^k draws.
-constexpr int kInitFrameBits = 31, kInitLaneTables = 6, kInitGroupBits = 22;
+// the bits of the group index; before them the frame bits, 2^32 2^k draws.
+// Partly filled blocks count whole, so an image one pixel wide has the most for
+// its pixels, one per four, and eight times fewer groups.
+constexpr int64_t kMaxImagePixels = int64_t(1) << 28;   // larger images are refused
+constexpr int kInitFrameBits = 31, kInitLaneTables = 6, kInitGroupBits = 23;
+static_assert((kMaxImagePixels / 4 / 8 - 1) >> kInitGroupBits == 0, "every group index has its tables");
 constexpr int kInitTables = kInitFrameBits + kInitLaneTables + kInitGroupBits;
 inline std::vector<uint32_t> xorwow_init_tables()
 {
