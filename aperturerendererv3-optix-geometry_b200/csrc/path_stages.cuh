@@ -19,17 +19,19 @@ namespace ar {
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 __device__ __forceinline__ unsigned lanes_below() { return (1u << lane_id()) - 1u; }
 
-// Warp-aggregated allocation: one atomic per warp, indices ordered by lane.
-// Returns the caller's index, or -1 when pred is false.
+// Warp-aggregated allocation, called by all 32 lanes together: one atomic per
+// warp, so the indices given out are consecutive, ordered by lane.  Returns the
+// caller's index, or -1 when pred is false.  (The mask is the whole warp, not
+// __activemask(), which may see only part of a warp that a branch has split:
+// k_shade stores the warp's records as one run of slots.)
 __device__ __forceinline__ int warp_alloc(int32_t* counter, bool pred)
 {
-    const unsigned active = __activemask();
-    const unsigned m = __ballot_sync(active, pred);
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, pred);
     if (m == 0) return -1;
     const int leader = __ffs(m) - 1;
     int base = 0;
     if (static_cast<int>(lane_id()) == leader) base = atomicAdd(counter, __popc(m));
-    base = __shfl_sync(active, base, leader);
+    base = __shfl_sync(0xFFFFFFFFu, base, leader);
     return pred ? base + __popc(m & lanes_below()) : -1;
 }
 
