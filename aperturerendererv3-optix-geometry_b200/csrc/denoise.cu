@@ -146,6 +146,7 @@ __device__ uint32_t stage_tstat(float4* w, int p, const ar_screen_stats* st, int
     const float fnum = static_cast<float>(s.num);
     const float fnm1 = static_cast<float>(max(s.num - 1u, 1u));
     float th[3], vth[3], u[3], l[3];
+    bool plain = true;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const float vb = static_cast<float>(static_cast<double>(s.m2_div_n[c]) * num * invNm1);
@@ -153,17 +154,17 @@ __device__ uint32_t stage_tstat(float4* w, int p, const ar_screen_stats* st, int
         th[c] = s.mean[c] + s.m3_div_n[c] / 6.0f / vb;
         u[c] = vb / fnum;
         l[c] = u[c] * u[c] / fnm1;
+        plain &= vb == 0.0f || (u[c] >= 1.0e-15f && u[c] <= 1.0e15f);
     }
     w[p] = make_float4(th[0], th[1], vth[0], vth[1]);
     w[kWin + p] = make_float4(u[0], u[1], l[0], l[1]);
     reinterpret_cast<float2*>(w + 2 * kWin)[p] = make_float2(th[2], vth[2]);
     reinterpret_cast<float2*>(w + 2 * kWin)[kWin + p] = make_float2(u[2], l[2]);
-    // sample count for the tile's bounds of nu; 1 where their derivation does
-    // not hold (a variance so small or large that its square leaves the float
-    // range); a zero variance makes theta infinite or NaN, so its taps fail
-    bool plain = true;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) plain &= u[c] == 0.0f ? vth[c] == 0.0f : u[c] >= 1.0e-15f && u[c] <= 1.0e15f;
+    // sample count for the tile's bounds of nu; 0 where their derivation does
+    // not hold: a variance so small or large that its square leaves the float
+    // range, or so small that its quotient u is zero, when a pair's nu may be
+    // 0 / 0.  A variance of exactly zero makes theta infinite or NaN, so its
+    // taps fail whatever nu is.
     return plain ? s.num : 0u;
 }
 
