@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/aperture_b200.h"
+#include "path_memory.h"
 #include "render_kernels.h"
 #include "scene_build.h"
 #include "sdf.cuh"
@@ -112,62 +113,18 @@ constexpr int64_t kMaxPool = int64_t(1) << 23;
 // 147,456 594 / 628 against 506 / 779.
 int tail_limit(int sm_count) { return 4 * sm_count * ar::kTailBlock; }
 
-// Path state of large renders: one block per device, lent to a render for its
-// duration, so scenes that render in turn share it.  A render that finds it lent
-// out allocates a block of its own; of the blocks that come back one is kept, the
-// larger, and it is freed with the device's last scene.  (A stream-ordered memory
-// pool did the same but took 25 ms longer to grow to 3.6 GB than cudaMalloc.)
-class PathMemory {
-public:
-    static void add_scene(int device)
+// Path state of large renders: PathMemory's blocks.
+struct DeviceMemory {
+    static void* alloc(size_t bytes)
     {
-        std::lock_guard<std::mutex> g(lock());
-        ++entries()[device].scenes;
-    }
-    static void remove_scene(int device)
-    {
-        std::lock_guard<std::mutex> g(lock());
-        Entry& e = entries()[device];
-        if (--e.scenes > 0) return;
-        if (e.mem) cudaFree(e.mem);
-        e.mem = nullptr;
-        e.bytes = 0;
-    }
-    // at least `bytes` (set to the block's size) on the current device, or NULL
-    static char* take(int device, size_t& bytes)
-    {
-        {
-            std::lock_guard<std::mutex> g(lock());
-            Entry& e = entries()[device];
-            if (e.mem && e.bytes >= bytes) {
-                char* p = e.mem;
-                bytes = e.bytes;
-                e.mem = nullptr;
-                return p;
-            }
-            if (e.mem) cudaFree(e.mem);   // too small: its successor comes back instead
-            e.mem = nullptr;
-        }
         void* p = nullptr;
-        if (cudaMalloc(&p, bytes) == cudaSuccess) return static_cast<char*>(p);
+        if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
         cudaGetLastError();
         return nullptr;
     }
-    static void give(int device, char* p, size_t bytes)   // idle: its last kernel has finished
-    {
-        std::lock_guard<std::mutex> g(lock());
-        Entry& e = entries()[device];
-        if (e.scenes > 0 && (!e.mem || e.bytes < bytes)) {
-            std::swap(p, e.mem);
-            e.bytes = bytes;
-        }
-        if (p) cudaFree(p);
-    }
-private:
-    struct Entry { char* mem = nullptr; size_t bytes = 0; int scenes = 0; };
-    static std::mutex& lock() { static std::mutex m; return m; }
-    static std::map<int, Entry>& entries() { static std::map<int, Entry> e; return e; }
+    static void free(void* p) { cudaFree(p); }
 };
+using PathMemory = ar::PathMemory<DeviceMemory>;
 
 // Lays the path state of `pool` paths out at b; returns its size (b may be NULL
 // to ask for it).
