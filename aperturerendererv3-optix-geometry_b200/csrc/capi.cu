@@ -106,12 +106,23 @@ private:
 // 2^20 / 2^21 paths, and per 64 samples 145.0 / 132.7 / 125.3 / 122.7 ms at
 // 2^21 / 2^22 / 2^23 / 2^24; 2^24 would take 7.2 GB for the last 2 %.
 constexpr int64_t kMaxPool = int64_t(1) << 23;
-// Paths left at which k_tail takes over from the wavefront: four for each of its
-// lanes (151,552).  One-sample images of box / sphere scene, microseconds by the
-// tail kernel against the wavefront: 64,000 pixels 335 / 400 against 395 / 708,
-// 76,800 383 / 450 against 415 / 750, 120,000 572 / 526 against 508 / 792,
-// 147,456 594 / 628 against 506 / 779.
-int tail_limit(int sm_count) { return 4 * sm_count * ar::kTailBlock; }
+// Paths left at which k_tail takes over from the wavefront, in paths for each of
+// its lanes: four (151,552) in scenes of triangles, cubes and spheres.  One-sample
+// images of box / sphere scene, microseconds by the tail kernel against the
+// wavefront: 64,000 pixels 335 / 400 against 395 / 708, 76,800 383 / 450 against
+// 415 / 750, 120,000 572 / 526 against 508 / 792, 147,456 594 / 628 against
+// 506 / 779.  SDF marches and tracking in a medium take lanes of a warp unequal
+// times, which the wavefront's kernels for them bound at one segment: two there,
+// and one with four wavelengths, whose shading is four times as long.  Box with
+// SDF tori and a medium, depth 12, limits of 1 / 2 / 4: RGB 38,400 pixels
+// 1365 / 940 / 945, 60,000 1474 / 1470 / 1471, 144,400 2087 / 2094 / 4041; four
+// wavelengths 38,400 2199 / 2048 / 2037, 60,000 2598 / 2983 / 2997, 144,400
+// 3215 / 3818 / 9051 (wavefront alone 3406).
+int tail_limit(const ar::SceneView& v, int spectral, int sm_count)
+{
+    const int per_lane = v.num_sdf == 0 && !v.has_medium ? 4 : spectral == 4 ? 1 : 2;
+    return per_lane * sm_count * ar::kTailBlock;
+}
 
 // Path state of large renders: PathMemory's blocks.
 struct DeviceMemory {
@@ -471,7 +482,7 @@ ar_status run_render(ar_scene* s, const ar_camera* cam, const ar_render_params* 
     int64_t launches = 2;
     const int grid_trace = s->grid_trace;
     const int grid_other = s->sm_count * 4;
-    const int tail = tail_limit(s->sm_count);
+    const int tail = tail_limit(s->view, fp.spectral, s->sm_count);
     LaunchTimers tm;
     LaunchTimers* tmp = stats ? &tm : nullptr;
     constexpr int kBatch = 16;
@@ -1268,7 +1279,7 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
                                  w.ovf, w.err, w.accum, nullptr, K, &w.cur, gt, go, w.st, &launches, nullptr),
            "capture iterations");
         ck(ar::launch_tail(jb.scene->view, w.fp, w.B, w.ctl, w.stats, w.ovf, w.err, w.accum, nullptr, w.cur,
-                           tail_limit(jb.scene->sm_count), jb.scene->sm_count, w.st), "capture tail");
+                           tail_limit(jb.scene->view, w.fp.spectral, jb.scene->sm_count), jb.scene->sm_count, w.st), "capture tail");
         ++launches;
         ck(cudaEventRecord(w.done, w.st), "join");
         ck(cudaStreamWaitEvent(st, w.done, 0), "join");
