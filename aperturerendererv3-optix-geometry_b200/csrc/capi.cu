@@ -126,6 +126,7 @@ int tail_limit(const ar::SceneView& v, int spectral, int sm_count)
 
 // Path state of large renders: PathMemory's blocks.
 struct DeviceMemory {
+    static constexpr size_t kKeep = size_t(4) << 30;
     static void* alloc(size_t bytes)
     {
         void* p = nullptr;

@@ -1,21 +1,25 @@
 // path_memory.h -- the blocks of device memory that hold path state, kept
 // between calls and shared by the scenes of a device.  Memory is the allocator:
-// static void* alloc(size_t), NULL when there is none, and static void free(void*),
-// both for the current device.
+// static void* alloc(size_t), NULL when there is none, static void free(void*),
+// both for the current device, and kKeep, the size of the largest block kept.
 #pragma once
 
 #include <cstddef>
+#include <iterator>
 #include <map>
 #include <mutex>
-#include <utility>
 
 namespace ar {
 
-// One block per device, lent to a call for its duration, so scenes that render in
-// turn share it.  A call that finds it lent out allocates a block of its own; of
-// the blocks that come back one is kept, the larger, and it is freed with the
-// device's last scene.  (A stream-ordered memory pool did the same but took 25 ms
-// longer to grow to 3.6 GB than cudaMalloc.)
+// A block is lent to a call for its duration, so scenes that render in turn share
+// one.  A call that finds none idle that is large enough allocates; the largest
+// idle block then gives way, as the new one will come back in its place.  So a
+// device holds as many blocks as calls have run on it at once, and no more than
+// it has scenes: with one block for all, two threads that rendered at the same
+// time allocated and freed 3.6 GB on every call.  Blocks above Memory::kKeep bytes
+// are not kept, and the last scene of the device frees them all.  (A
+// stream-ordered memory pool did the same but took 25 ms longer to grow to 3.6 GB
+// than cudaMalloc.)
 template <class Memory>
 class PathMemory {
 public:
@@ -26,42 +30,52 @@ public:
     }
     static void remove_scene(int device)
     {
-        std::lock_guard<std::mutex> g(lock());
-        Entry& e = entries()[device];
-        if (--e.scenes > 0) return;
-        if (e.mem) Memory::free(e.mem);
-        e.mem = nullptr;
-        e.bytes = 0;
+        std::multimap<size_t, void*> gone;
+        {
+            std::lock_guard<std::mutex> g(lock());
+            Entry& e = entries()[device];
+            if (--e.scenes > 0) return;
+            gone.swap(e.idle);
+        }
+        for (auto& b : gone) Memory::free(b.second);
     }
     // at least `bytes` (set to the block's size) on the current device, or NULL
     static char* take(int device, size_t& bytes)
     {
+        void* gone = nullptr;
         {
             std::lock_guard<std::mutex> g(lock());
-            Entry& e = entries()[device];
-            if (e.mem && e.bytes >= bytes) {
-                char* p = e.mem;
-                bytes = e.bytes;
-                e.mem = nullptr;
+            auto& idle = entries()[device].idle;
+            auto fit = idle.lower_bound(bytes);
+            if (fit != idle.end()) {
+                char* p = static_cast<char*>(fit->second);
+                bytes = fit->first;
+                idle.erase(fit);
                 return p;
             }
-            if (e.mem) Memory::free(e.mem);   // too small: its successor comes back instead
-            e.mem = nullptr;
+            if (!idle.empty()) {
+                auto last = std::prev(idle.end());
+                gone = last->second;
+                idle.erase(last);
+            }
         }
+        if (gone) Memory::free(gone);
         return static_cast<char*>(Memory::alloc(bytes));
     }
     static void give(int device, char* p, size_t bytes)   // idle: its last kernel has finished
     {
-        std::lock_guard<std::mutex> g(lock());
-        Entry& e = entries()[device];
-        if (e.scenes > 0 && (!e.mem || e.bytes < bytes)) {
-            std::swap(p, e.mem);
-            e.bytes = bytes;
+        {
+            std::lock_guard<std::mutex> g(lock());
+            Entry& e = entries()[device];
+            if (bytes <= Memory::kKeep && static_cast<int>(e.idle.size()) < e.scenes) {
+                e.idle.emplace(bytes, p);
+                return;
+            }
         }
-        if (p) Memory::free(p);
+        Memory::free(p);
     }
 private:
-    struct Entry { char* mem = nullptr; size_t bytes = 0; int scenes = 0; };
+    struct Entry { std::multimap<size_t, void*> idle; int scenes = 0; };   // blocks by size
     // never destroyed: scenes owned by objects with static storage are released
     // during process exit, after the destructors of what was first used later
     static std::mutex& lock() { static std::mutex* m = new std::mutex; return *m; }

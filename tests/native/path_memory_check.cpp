@@ -9,6 +9,7 @@
 #include "../../aperturerendererv3-optix-geometry_b200/csrc/path_memory.h"
 
 struct Fake {
+    static constexpr size_t kKeep = 500;
     static std::map<void*, size_t>& live() { static auto* m = new std::map<void*, size_t>; return *m; }
     static size_t room;   // bytes that may be live at once
     static int allocs;
@@ -62,9 +63,59 @@ int at_exit()
     return 0;   // "OK" comes from the owner's destructor
 }
 
+// Calls in turn share one block; it grows with the largest.
+int in_turn()
+{
+    Blocks::add_scene(0);
+    Blocks::add_scene(0);
+    for (size_t need : {100, 60, 100, 200, 30, 200}) {
+        size_t n = need;
+        char* p = Blocks::take(0, n);
+        CHECK(p && n >= need);
+        CHECK(Fake::live().size() == 1);
+        Blocks::give(0, p, n);
+    }
+    CHECK(Fake::allocs == 2 && Fake::used() == 200);
+    Blocks::remove_scene(0);
+    CHECK(Fake::live().size() == 1);
+    Blocks::remove_scene(0);
+    CHECK(Fake::live().empty());
+    return std::printf("OK\n"), 0;
+}
+
+// Calls at once keep a block each, of their own size, and allocate no more.
+int at_once()
+{
+    for (int k = 0; k < 2; ++k) Blocks::add_scene(3);
+    for (int round = 0; round < 4; ++round) {
+        size_t a = 100, b = 40;
+        char *p = Blocks::take(3, a), *q = Blocks::take(3, b);
+        CHECK(p && q && p != q && a == 100 && b == 40);
+        Blocks::give(3, q, b);
+        Blocks::give(3, p, a);
+        CHECK(Fake::allocs == 2 && Fake::live().size() == 2);
+    }
+    // a third at once: only as many blocks as scenes are kept
+    size_t n[3] = {100, 40, 30};
+    char* r[3];
+    for (int k = 0; k < 3; ++k) r[k] = Blocks::take(3, n[k]);
+    for (int k = 0; k < 3; ++k) Blocks::give(3, r[k], n[k]);
+    CHECK(Fake::live().size() == 2);
+    size_t big = 501;   // above kKeep
+    char* p = Blocks::take(3, big);
+    CHECK(p);
+    Blocks::give(3, p, big);
+    CHECK(Fake::used() <= 500);
+    for (int k = 0; k < 2; ++k) Blocks::remove_scene(3);
+    CHECK(Fake::live().empty());
+    return std::printf("OK\n"), 0;
+}
+
 int main(int argc, char** argv)
 {
     const char* what = argc > 1 ? argv[1] : "";
     if (!std::strcmp(what, "exit")) return at_exit();
+    if (!std::strcmp(what, "in_turn")) return in_turn();
+    if (!std::strcmp(what, "at_once")) return at_once();
     return 2;
 }
