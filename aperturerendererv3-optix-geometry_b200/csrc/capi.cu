@@ -25,6 +25,10 @@
 #include "sdf.cuh"
 #include "xorwow_jump.h"
 
+namespace ar {
+bool release_idle_memory();
+}
+
 namespace {
 
 thread_local std::string g_last_error;
@@ -49,12 +53,31 @@ void ck(cudaError_t e, const char* where)
     }
 }
 
+// Path state of large renders and batches: blocks of device memory kept between
+// calls (path_memory.h).
+struct DeviceMemory {
+    static constexpr size_t kKeep = size_t(4) << 30;
+    static void* alloc(size_t bytes)
+    {
+        void* p = nullptr;
+        if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+        cudaGetLastError();
+        return nullptr;
+    }
+    static void free(void* p) { cudaFree(p); }
+};
+using PathMemory = ar::PathMemory<DeviceMemory>;
+
 template <class T>
 T* dalloc(size_t count, const char* what)
 {
     if (count == 0) count = 1;
     void* p = nullptr;
-    const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+    cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+    if (e == cudaErrorMemoryAllocation && ar::release_idle_memory()) {
+        cudaGetLastError();
+        e = cudaMalloc(&p, count * sizeof(T));
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         throw CudaError(e, std::string("cudaMalloc ") + what);
@@ -124,20 +147,6 @@ int tail_limit(const ar::SceneView& v, int spectral, int sm_count)
     return per_lane * sm_count * ar::kTailBlock;
 }
 
-// Path state of large renders: PathMemory's blocks.
-struct DeviceMemory {
-    static constexpr size_t kKeep = size_t(4) << 30;
-    static void* alloc(size_t bytes)
-    {
-        void* p = nullptr;
-        if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
-        cudaGetLastError();
-        return nullptr;
-    }
-    static void free(void* p) { cudaFree(p); }
-};
-using PathMemory = ar::PathMemory<DeviceMemory>;
-
 // Lays the path state of `pool` paths out at b; returns its size (b may be NULL
 // to ask for it).
 size_t path_layout(ar::PathBuffers& B, char* b, int64_t pool)
@@ -163,37 +172,21 @@ size_t path_layout(ar::PathBuffers& B, char* b, int64_t pool)
     return off;
 }
 
-// What a batch needs besides its graph, kept by the scene of its first job from
-// one batch to the next: the jobs' workspaces as one allocation (at most
-// kBatchKeep bytes are kept), and a stream and an event per job.  A second batch
-// that runs at the same time finds the lock taken and makes its own.
-constexpr size_t kBatchKeep = size_t(4) << 30;
-struct BatchArena {
+// A stream and an event per job of a batch, kept by the scene of its first job
+// from one batch to the next.  A second batch that runs at the same time finds
+// the lock taken and makes its own.  (The jobs' workspaces come from PathMemory.)
+struct BatchHandles {
     std::mutex lock;
-    char* mem = nullptr;
-    size_t bytes = 0;
     std::vector<cudaStream_t> streams;
     std::vector<cudaEvent_t> events;
     void clear()
     {
-        if (mem) cudaFree(mem);
-        mem = nullptr;
-        bytes = 0;
         for (cudaEvent_t e : events) cudaEventDestroy(e);
         for (cudaStream_t s : streams) cudaStreamDestroy(s);
         events.clear();
         streams.clear();
     }
-    void reserve(size_t need)
-    {
-        if (bytes >= need) return;
-        if (mem) cudaFree(mem);
-        mem = nullptr;
-        bytes = 0;
-        mem = dalloc<char>(need, "batch workspaces");
-        bytes = need;
-    }
-    void handles(size_t n)
+    void reserve(size_t n)
     {
         while (streams.size() < n) {
             cudaStream_t s;
@@ -254,7 +247,7 @@ struct ar_scene {
     int* err = nullptr;
     uint32_t* ovf = nullptr;  // traversal stack overflow slabs, one per persistent thread
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    BatchArena batch;   // of batches whose first job is this scene's
+    BatchHandles batch;   // of batches whose first job is this scene's
     std::vector<cudaEvent_t> timer_ext, timer_sh;  // event pairs around traversal launches
 
     ~ar_scene()
@@ -620,6 +613,13 @@ bool scene_view_of(const ar_scene* s, SceneView* v, int* device, int* sm_count)
     return true;
 }
 ar_status set_error(ar_status st, const std::string& msg) { return fail(st, msg); }
+// Frees what is kept on the current device between calls and not in use; whether there was any.
+bool release_idle_memory()
+{
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    return ::PathMemory::trim(device);
+}
 }  // namespace ar
 
 extern "C" {
@@ -1050,9 +1050,11 @@ __global__ void k_batch_drain(BatchDrain d, cudaGraphConditionalHandle h)
 
 struct BatchResources {
     std::vector<JobWs> jobs;
-    BatchArena own;                 // used when the scene's arena is taken
-    BatchArena* arena = nullptr;
+    BatchHandles own;               // used when the scene's are taken
     std::unique_lock<std::mutex> held;
+    int device = 0;
+    char* mem = nullptr;            // the jobs' workspaces: a block of PathMemory
+    size_t bytes = 0;
     cudaEvent_t fork = nullptr;
     cudaStream_t orch = nullptr;
     cudaGraph_t graph = nullptr;
@@ -1065,7 +1067,7 @@ struct BatchResources {
             cudaStreamEndCapture(orch, &g);
             cudaGetLastError();
         }
-        // also after an error: nothing of the batch may still use the arena
+        // also after an error: nothing of the batch may still use its workspaces
         if (orch) cudaStreamSynchronize(orch);
         for (JobWs& w : jobs)
             if (w.st) cudaStreamSynchronize(w.st);
@@ -1074,7 +1076,7 @@ struct BatchResources {
         if (fork) cudaEventDestroy(fork);
         if (orch) cudaStreamDestroy(orch);
         own.clear();
-        if (arena && arena != &own && arena->bytes > kBatchKeep) arena->clear();
+        if (mem) PathMemory::give(device, mem, bytes);
     }
 };
 
@@ -1193,33 +1195,41 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
     ck(cudaStreamWaitEvent(st, R.fork, 0), "order after caller");
     ck(cudaEventRecord(t0, st), "event record");
     ck(cudaEventRecord(R.fork, st), "event record");
-    size_t bytes = 0;
-    for (int j = 0; j < njobs; ++j) {
-        JobWs& w = R.jobs[j];
-        const ar_job& jb = jobs[j];
-        w.npix = static_cast<int64_t>(jb.camera.width) * jb.camera.height;
-        w.total = w.npix * jb.params.spp;
-        int64_t pool = static_cast<int64_t>(static_cast<double>(budget) * static_cast<double>(w.total) /
-                                            static_cast<double>(totalAll));
-        if (jb.params.wave_paths > 0) pool = jb.params.wave_paths;
-        pool = std::max<int64_t>(std::min<int64_t>(pool, kMaxPool), int64_t(1) << 14);
-        w.pool = std::max<int64_t>(1, std::min<int64_t>(pool, w.total));
-        w.fp = make_frame(jb.scene, &jb.camera, &jb.params);
-        w.fp.pool = static_cast<int32_t>(w.pool);
-        bytes += job_layout(w, nullptr, w.pool, w.npix, jb.scene->grid_trace);
-    }
     const size_t drain_bytes = static_cast<size_t>(njobs) * 16 + 64;
+    R.device = s0->device;
+    // when memory is short the pools are halved, down to the 2^14 paths that every
+    // job has in any case
+    for (int halvings = 0; !R.mem; ++halvings) {
+        bool least = true;
+        R.bytes = drain_bytes;
+        for (int j = 0; j < njobs; ++j) {
+            JobWs& w = R.jobs[j];
+            const ar_job& jb = jobs[j];
+            w.npix = static_cast<int64_t>(jb.camera.width) * jb.camera.height;
+            w.total = w.npix * jb.params.spp;
+            int64_t pool = static_cast<int64_t>(static_cast<double>(budget) * static_cast<double>(w.total) /
+                                                static_cast<double>(totalAll));
+            if (jb.params.wave_paths > 0) pool = jb.params.wave_paths;
+            pool = std::max<int64_t>(std::min<int64_t>(pool, kMaxPool) >> halvings, int64_t(1) << 14);
+            least = least && pool == int64_t(1) << 14;
+            w.pool = std::max<int64_t>(1, std::min<int64_t>(pool, w.total));
+            w.fp = make_frame(jb.scene, &jb.camera, &jb.params);
+            w.fp.pool = static_cast<int32_t>(w.pool);
+            R.bytes += job_layout(w, nullptr, w.pool, w.npix, jb.scene->grid_trace);
+        }
+        R.mem = PathMemory::take(R.device, R.bytes);
+        if (!R.mem && least) throw CudaError(cudaErrorMemoryAllocation, "cudaMalloc batch workspaces");
+    }
     R.held = std::unique_lock<std::mutex>(jobs[0].scene->batch.lock, std::try_to_lock);
-    R.arena = R.held.owns_lock() ? &jobs[0].scene->batch : &R.own;
-    R.arena->reserve(bytes + drain_bytes);
-    R.arena->handles(static_cast<size_t>(njobs));
-    char* next = R.arena->mem;
+    BatchHandles& handles = R.held.owns_lock() ? jobs[0].scene->batch : R.own;
+    handles.reserve(static_cast<size_t>(njobs));
+    char* next = R.mem;
     for (int j = 0; j < njobs; ++j) {
         JobWs& w = R.jobs[j];
         const ar_job& jb = jobs[j];
         next += job_layout(w, next, w.pool, w.npix, jb.scene->grid_trace);
-        w.st = R.arena->streams[static_cast<size_t>(j)];
-        w.done = R.arena->events[static_cast<size_t>(j)];
+        w.st = handles.streams[static_cast<size_t>(j)];
+        w.done = handles.events[static_cast<size_t>(j)];
         ck(cudaStreamWaitEvent(w.st, R.fork, 0), "fork");
         ck(ar::launch_rng_init(w.fp, w.base0, w.base1, jb.scene->init_tables, jb.scene->sm_count, w.st), "rng init");
         ck(ar::launch_render_init(w.ctl, w.total, w.accum, w.npix, w.stats, w.err, jb.scene->sm_count, w.st), "render init");

@@ -17,7 +17,8 @@ namespace ar {
 // device holds as many blocks as calls have run on it at once, and no more than
 // it has scenes: with one block for all, two threads that rendered at the same
 // time allocated and freed 3.6 GB on every call.  Blocks above Memory::kKeep bytes
-// are not kept, and the last scene of the device frees them all.  (A
+// are not kept, an allocation that finds no room has the idle ones freed and tries
+// again (trim), and the last scene of the device frees them all.  (A
 // stream-ordered memory pool did the same but took 25 ms longer to grow to 3.6 GB
 // than cudaMalloc.)
 template <class Memory>
@@ -60,7 +61,20 @@ public:
             }
         }
         if (gone) Memory::free(gone);
-        return static_cast<char*>(Memory::alloc(bytes));
+        void* p = Memory::alloc(bytes);
+        if (!p && trim(device)) p = Memory::alloc(bytes);
+        return static_cast<char*>(p);
+    }
+    // Frees the idle blocks, for an allocation that found no room; false if there were none.
+    static bool trim(int device)
+    {
+        std::multimap<size_t, void*> gone;
+        {
+            std::lock_guard<std::mutex> g(lock());
+            gone.swap(entries()[device].idle);
+        }
+        for (auto& b : gone) Memory::free(b.second);
+        return !gone.empty();
     }
     static void give(int device, char* p, size_t bytes)   // idle: its last kernel has finished
     {

@@ -13,6 +13,7 @@
 namespace ar {
 
 ar_status set_error(ar_status st, const std::string& msg);
+bool release_idle_memory();
 
 namespace {
 
@@ -65,8 +66,15 @@ extern "C" ar_status ar_tonemap(const float* rgb, size_t n, int32_t tone_type, f
     uint32_t* out = bgra;
     cudaError_t e = cudaSuccess;
     if (mem_kind == AR_MEM_HOST) {
-        if ((e = cudaMalloc(&tmp.rgb, n * 3 * sizeof(float))) != cudaSuccess) return cuda_fail(e, "cudaMalloc");
-        if ((e = cudaMalloc(&tmp.out, n * sizeof(uint32_t))) != cudaSuccess) return cuda_fail(e, "cudaMalloc");
+        for (int k = 0; k < 2; ++k) {
+            auto alloc = [&] { return k ? cudaMalloc(&tmp.out, n * sizeof(uint32_t)) : cudaMalloc(&tmp.rgb, n * 3 * sizeof(float)); };
+            e = alloc();
+            if (e == cudaErrorMemoryAllocation && release_idle_memory()) {
+                cudaGetLastError();
+                e = alloc();
+            }
+            if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc");
+        }
         if ((e = cudaMemcpyAsync(tmp.rgb, rgb, n * 3 * sizeof(float), cudaMemcpyHostToDevice, st)) != cudaSuccess)
             return cuda_fail(e, "cudaMemcpyAsync");
         in = tmp.rgb;

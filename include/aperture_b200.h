@@ -243,7 +243,14 @@ ar_status ar_bvh_build_info(const ar_object_desc* objects, size_t count, const a
  *   accum     width*height*3 doubles holding running sums, or NULL; when given it
  *             is ADDED to (resume/extend a render), never cleared
  *   mem_kind  AR_MEM_HOST or AR_MEM_DEVICE for both buffers
- *   stats     optional counters (NULL to skip)                                 */
+ *   stats     optional counters (NULL to skip)
+ * Memory kept between calls: per scene the pixel state of its largest image (60
+ * bytes a pixel) and the path state of small renders (up to 2^18 paths, 0.12 GB);
+ * per device the path state of larger renders and of batches, in blocks of up to
+ * 4 GiB (3.6 GB for 2^23 paths in flight), one for calls in turn, one more for
+ * each that runs at the same time, at most one per scene.  Calls of this library
+ * that find no room free the blocks not in use, renders and batches then run with
+ * fewer paths in flight, and the device's last scene frees them all.            */
 ar_status ar_render(ar_scene* scene, const ar_camera* camera, const ar_render_params* params,
                     float* out_rgb, double* accum, int32_t mem_kind, void* stream,
                     ar_render_stats* stats);

@@ -111,11 +111,34 @@ int at_once()
     return std::printf("OK\n"), 0;
 }
 
+// Where memory is short the idle blocks give way.
+int pressure()
+{
+    for (int k = 0; k < 3; ++k) Blocks::add_scene(0);
+    size_t n[3] = {100, 120, 130};
+    char* p[3];
+    for (int k = 0; k < 3; ++k) p[k] = Blocks::take(0, n[k]);
+    for (int k = 0; k < 3; ++k) Blocks::give(0, p[k], n[k]);
+    CHECK(Fake::used() == 350);
+    Fake::room = 400;
+    size_t big = 390;   // fits only without all three
+    char* q = Blocks::take(0, big);
+    CHECK(q && Fake::used() == 390);
+    size_t more = 20;   // no room, nothing idle
+    CHECK(!Blocks::take(0, more));
+    Blocks::give(0, q, big);
+    CHECK(!Blocks::trim(1) && Fake::used() == 390);
+    CHECK(Blocks::trim(0) && Fake::live().empty() && !Blocks::trim(0));
+    for (int k = 0; k < 3; ++k) Blocks::remove_scene(0);
+    return std::printf("OK\n"), 0;
+}
+
 int main(int argc, char** argv)
 {
     const char* what = argc > 1 ? argv[1] : "";
     if (!std::strcmp(what, "exit")) return at_exit();
     if (!std::strcmp(what, "in_turn")) return in_turn();
     if (!std::strcmp(what, "at_once")) return at_once();
+    if (!std::strcmp(what, "pressure")) return pressure();
     return 2;
 }

@@ -18,9 +18,10 @@ def check(tmp_path_factory):
 
 
 @pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
-@pytest.mark.parametrize("what", ["exit", "in_turn", "at_once"])
+@pytest.mark.parametrize("what", ["exit", "in_turn", "at_once", "pressure"])
 def test_kept_blocks(check, what):
     """exit: a scene released by a static object's destructor finds the blocks' records still there.
-    in_turn: one block serves calls one after the other.  at_once: calls at the same time keep a block each."""
+    in_turn: one block serves calls one after the other.  at_once: calls at the same time keep a block each.
+    pressure: the idle blocks give way where memory is short."""
     out = subprocess.run([str(check), what], capture_output=True, text=True, timeout=60)
     assert out.returncode == 0 and out.stdout.strip() == "OK", out.stdout + out.stderr[:2000]

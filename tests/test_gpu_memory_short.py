@@ -1,0 +1,71 @@
+"""Calls where little device memory is left: what earlier calls kept gives way,
+and batches run with fewer paths in flight, as single renders do."""
+import numpy as np
+import pytest
+
+import scenes
+from aperture_b200 import Scene, make_params, render_batch
+
+GIB = 1 << 30
+
+
+class Short:
+    """All but `leave` bytes of the device's free memory, held while inside."""
+    def __init__(self, leave):
+        self.leave = int(leave)
+
+    def __enter__(self):
+        import torch
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free, _ = torch.cuda.mem_get_info()
+        self.held = torch.empty(free - self.leave, dtype=torch.uint8, device="cuda")
+
+    def __exit__(self, *exc):
+        import torch
+        del self.held
+        torch.cuda.empty_cache()
+
+
+def device_image(scene, cam, out, **par):
+    import torch
+    scene.render_device(cam, make_params(**par), out.data_ptr())
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+@pytest.mark.gpu
+def test_batch_with_little_memory(box_objects):
+    """8.4 million paths: the default share of paths in flight takes 3.7 GB."""
+    import torch
+    scene = Scene(box_objects)
+    outs = [torch.zeros(700 * 500 * 3, device="cuda") for _ in range(3)]
+    jobs = [(scene, scenes.box_camera(700, 500), make_params(spp=8, max_depth=4, frame_offset=8 * k), o.data_ptr(), None)
+            for k, o in enumerate(outs)]
+    render_batch(jobs, path_budget=1 << 16)
+    torch.cuda.synchronize()
+    ref = [o.cpu().numpy() for o in outs]
+    [o.zero_() for o in outs]
+    with Short(2.5 * GIB):
+        st = render_batch(jobs)
+        torch.cuda.synchronize()
+    assert st.paths == 3 * 700 * 500 * 8
+    for o, r in zip(outs, ref):
+        np.testing.assert_allclose(o.cpu().numpy(), r, rtol=1e-6, atol=1e-7)
+
+
+@pytest.mark.gpu
+def test_kept_memory_gives_way(box_objects):
+    """A large render leaves its path state (3.6 GB) behind; a larger image in
+    another scene needs that room."""
+    import torch
+    first, second = Scene(box_objects), Scene(box_objects)
+    small, large = torch.zeros(1920 * 1080 * 3, device="cuda"), torch.zeros(4096 * 4096 * 3, device="cuda")
+    ref = device_image(first, scenes.box_camera(4096, 4096), large, spp=1, max_depth=3)
+    first.close()
+    first = Scene(box_objects)
+    device_image(first, scenes.box_camera(1920, 1080), small, spp=5, max_depth=3)
+    large.zero_()
+    with Short(0.8 * GIB):
+        got = device_image(second, scenes.box_camera(4096, 4096), large, spp=1, max_depth=3)
+    assert np.array_equal(got, ref)
