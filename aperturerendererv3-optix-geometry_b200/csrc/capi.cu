@@ -309,12 +309,30 @@ private:
     cudaStream_t st_;
 };
 
+// Frees the workspace; nothing of the scene points into it afterwards, so the
+// scene stays usable when its successor cannot be allocated.
+void drop_workspace(ar_scene* s)
+{
+    if (s->ws) cudaFree(s->ws);
+    s->ws = nullptr;
+    s->ws_pix = 0;
+    s->rng_valid = false;
+    s->base0 = nullptr;
+    s->base1 = nullptr;
+    s->accum = nullptr;
+    s->fout = nullptr;
+    s->ctl = nullptr;
+    s->stats = nullptr;
+    s->err = nullptr;
+    s->ovf = nullptr;
+}
+
 // Carve the per-pixel buffers and counters from one allocation (re-used across
 // calls; grown when a larger image comes).
 void ensure_workspace(ar_scene* s, int64_t npix)
 {
     if (s->ws && s->ws_pix >= npix) return;
-    if (s->ws) { cudaFree(s->ws); s->ws = nullptr; }
+    drop_workspace(s);
     size_t off = 0;
     auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
     const size_t N = static_cast<size_t>(npix);
@@ -323,7 +341,6 @@ void ensure_workspace(ar_scene* s, int64_t npix)
     const size_t o_ovf = take(static_cast<size_t>(s->grid_trace) * ar::kTraceBlock * ar::kStackOverflow * 4);
     s->ws = dalloc<char>(off, "render workspace");
     s->ws_pix = npix;
-    s->rng_valid = false;
     char* b = s->ws;
     s->base0 = reinterpret_cast<uint4*>(b + o_b0);
     s->base1 = reinterpret_cast<uint2*>(b + o_b1);
@@ -1386,7 +1403,7 @@ ar_status ar_trace_rays(ar_scene* s, const float* rays, size_t n, int32_t any_hi
     AR_GUARD_BEGIN
     DeviceGuard g(s->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (!s->err) ensure_workspace(s, 1);
+    ensure_workspace(s, 1);
     ck(cudaMemsetAsync(s->err, 0, 64, st), "memset err");
     const float4* drays;
     int32_t* dobj;

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import scenes
-from aperture_b200 import Scene, make_params, render_batch
+from aperture_b200 import ArError, Scene, make_params, render_batch
 
 GIB = 1 << 30
 
@@ -69,3 +69,29 @@ def test_kept_memory_gives_way(box_objects):
     with Short(0.8 * GIB):
         got = device_image(second, scenes.box_camera(4096, 4096), large, spp=1, max_depth=3)
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.gpu
+def test_scene_after_an_image_that_did_not_fit(box_objects):
+    """A render whose per-pixel state (8 GB) finds no room; the scene's ray
+    queries and renders go on."""
+    import torch
+    scene = Scene(box_objects)
+    out = torch.zeros(64 * 48 * 3, device="cuda")
+    ref = device_image(scene, scenes.box_camera(64, 48), out, spp=2, max_depth=5)
+    rng = np.random.default_rng(6)
+    rays = np.zeros((500, 8), np.float32)
+    rays[:, :3] = rng.uniform(-0.4, 0.4, (500, 3))
+    rays[:, 4:7] = rng.normal(size=(500, 3))
+    rays[:, 4:7] /= np.linalg.norm(rays[:, 4:7], axis=1, keepdims=True)
+    rays[:, 7] = 1e30
+    hits, t = scene.trace_rays(rays)
+    huge = torch.zeros(16384 * 8192 * 3, device="cuda")
+    with Short(1.5 * GIB):
+        with pytest.raises(ArError, match="OUT_OF_MEMORY"):
+            scene.render_device(scenes.box_camera(16384, 8192), make_params(spp=1, max_depth=2), huge.data_ptr())
+        again, ta = scene.trace_rays(rays)
+        out.zero_()
+        img = device_image(scene, scenes.box_camera(64, 48), out, spp=2, max_depth=5)
+    assert np.array_equal(again, hits) and np.array_equal(ta, t)
+    np.testing.assert_allclose(img, ref, rtol=1e-6, atol=1e-7)
