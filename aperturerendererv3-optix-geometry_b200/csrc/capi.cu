@@ -1571,6 +1571,8 @@ void nrc_ensure_queries(ar_nrc* c, int64_t n)
     for (auto it = c->owned.begin(); it != c->owned.end(); ++it)
         if (*it == c->queries) { c->owned.erase(it); break; }
     if (c->queries) cudaFree(c->queries);
+    c->queries = nullptr;   // and stays so if the allocation fails
+    c->query_cap = 0;
     c->queries = nrc_alloc<ar::NrcQuery>(c, static_cast<size_t>(n), "cache queries");
     c->query_cap = n;
 }
@@ -2056,6 +2058,7 @@ void guide_ensure_frame(ar_guide* g, int64_t npix)
     if (npix <= g->npix) return;
     for (void* p : g->frame_bufs) cudaFree(p);
     g->frame_bufs.clear();
+    g->npix = 0;   // and stays so if an allocation fails
     const size_t n = static_cast<size_t>(npix);
     g->view.events = guide_alloc<float4>(g->frame_bufs, n * ar::kPgEvents * 3, "guiding events");
     g->view.event_lb = guide_alloc<float4>(g->frame_bufs, n * ar::kPgEvents, "guiding events");

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import scenes
-from aperture_b200 import ArError, Scene, make_params, render_batch
+from aperture_b200 import ArError, PathGuide, RadianceCache, Scene, make_params, nrc_config, render_batch
 
 GIB = 1 << 30
 
@@ -95,3 +95,37 @@ def test_scene_after_an_image_that_did_not_fit(box_objects):
         img = device_image(scene, scenes.box_camera(64, 48), out, spp=2, max_depth=5)
     assert np.array_equal(again, hits) and np.array_equal(ta, t)
     np.testing.assert_allclose(img, ref, rtol=1e-6, atol=1e-7)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", ["cache", "guide"])
+def test_frames_after_one_that_did_not_fit(box_objects, what):
+    """A cache's queries (10 GB) and a guide's events (more) find no room; the next
+    frames are those of an object of the same history without that frame."""
+    import torch
+    scene = Scene(box_objects)
+    out, huge = torch.zeros(64 * 48 * 3, device="cuda"), torch.zeros(16384 * 8192 * 3, device="cuda")
+
+    def frame(on, w, h, f, to):
+        par = make_params(spp=1, max_depth=5, frame_offset=f)
+        if what == "cache":
+            on.render_frame(scenes.box_camera(w, h), par, to.data_ptr(), None, train=False)
+        else:
+            on.render_frame(scenes.box_camera(w, h), par, to.data_ptr(), None)
+        torch.cuda.synchronize()
+        return to[:w * h * 3].cpu().numpy()
+
+    def start():   # a first frame, so that there is something to outgrow
+        on = RadianceCache(scene, nrc_config(log2_entries=10, train_paths=64)) if what == "cache" else PathGuide(scene)
+        frame(on, 64, 48, 9, out)
+        return on
+    ref = frame(start(), 64, 48, 0, out)
+    on = start()
+    with Short(1.5 * GIB):
+        with pytest.raises(ArError, match="OUT_OF_MEMORY"):
+            frame(on, 16384, 8192, 0, huge)
+        got = frame(on, 64, 48, 0, out)
+    if what == "cache":
+        np.testing.assert_allclose(got, ref, rtol=1e-6, atol=1e-7)
+    else:   # the probes' sums depend on the order of additions
+        assert abs(got.mean() / ref.mean() - 1) < 0.02
