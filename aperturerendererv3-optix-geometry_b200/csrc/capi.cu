@@ -208,8 +208,7 @@ struct ar_scene {
     int sm_count = 148;
     ar::SceneView view{};
     int grid_trace = 0;
-    const uint32_t* jump_table = nullptr;  // A^(2^32) lookup table of the XORWOW register
-    const uint32_t* init_tables = nullptr;   // xorwow_init_tables(): the jumps of the per-pixel initialisation
+    const uint32_t* rng_tables = nullptr;    // xorwow_init_tables(), the device's copy; the first is the frame jump
     int64_t objects = 0, triangles = 0, lights = 0, nodes = 0, prims = 0;
     int64_t device_bytes = 0;
     std::vector<void*> owned;
@@ -487,7 +486,7 @@ ar_status run_render(ar_scene* s, const ar_camera* cam, const ar_render_params* 
     // seed and image) starts from the states the previous one left.
     if (!(s->rng_valid && s->rng_seed == fp.seed && s->rng_width == fp.width && s->rng_height == fp.height &&
           s->rng_next_frame == fp.frame0))
-        ck(launch_rng_init(fp, s->base0, s->base1, s->init_tables, s->sm_count, st), "rng init");
+        ck(launch_rng_init(fp, s->base0, s->base1, s->rng_tables, s->sm_count, st), "rng init");
     s->rng_valid = false;
     ck(launch_render_init(s->ctl, total, s->accum, npix, s->stats, s->err, s->sm_count, st), "render init");
     int64_t launches = 2;
@@ -502,7 +501,7 @@ ar_status run_render(ar_scene* s, const ar_camera* cam, const ar_render_params* 
     if (total <= tail && pool == total) {
         // few paths, all in one wave: they start at once and k_tail runs them to their
         // end, with nothing to wait for in between
-        ck(launch_generate(fp, B, s->ctl, s->base0, s->base1, s->jump_table, rec_dev, cur, grid_other, st), "render launch");
+        ck(launch_generate(fp, B, s->ctl, s->base0, s->base1, s->rng_tables, rec_dev, cur, grid_other, st), "render launch");
         ck(launch_tail(s->view, fp, B, s->ctl, s->stats, s->ovf, s->err, s->accum, rec_dev, cur, tail, s->sm_count, st),
            "render launch");
         launches += 3;
@@ -530,7 +529,7 @@ ar_status run_render(ar_scene* s, const ar_camera* cam, const ar_render_params* 
                 tm.shadow_ev = s->timer_sh.data();
                 tm.cap = static_cast<int>(need / 2);
             }
-            ck(launch_iterations(s->view, fp, B, s->ctl, s->base0, s->base1, s->jump_table, s->stats, s->ovf, s->err,
+            ck(launch_iterations(s->view, fp, B, s->ctl, s->base0, s->base1, s->rng_tables, s->stats, s->ovf, s->err,
                                  s->accum, rec_dev, batch, &cur, grid_trace, grid_other, st, &launches, tmp),
                "render launch");
             ck(launch_tail(s->view, fp, B, s->ctl, s->stats, s->ovf, s->err, s->accum, rec_dev, cur, tail, s->sm_count, st),
@@ -699,12 +698,7 @@ ar_status ar_scene_create_ex(const ar_object_desc* objects, size_t count, const 
         v.light_object = static_cast<const int32_t*>(own(upload(hs.light_object, "lights"), hs.light_object.size() * 4));
         v.light_prob = static_cast<const float*>(own(upload(hs.light_prob, "lights"), hs.light_prob.size() * 4));
         v.light_tri = static_cast<const float4*>(own(upload(hs.light_tri, "light triangles"), hs.light_tri.size() * 16));
-        {
-            static const std::vector<uint32_t> jt = ar::xorwow_jump_table_2p32();
-            s->jump_table = static_cast<const uint32_t*>(own(upload(jt, "rng jump table"), jt.size() * 4));
-            static const std::vector<uint32_t> js = ar::xorwow_init_tables();
-            s->init_tables = static_cast<const uint32_t*>(own(upload(js, "rng jump tables"), js.size() * 4));
-        }
+        ck(ar::rng_tables(&s->rng_tables), "rng jump tables");
         {
             // SDF volumes, then the SDF records pointing at them (device and host copies)
             std::vector<const void*> vdev(hs.volumes.size());
@@ -1248,7 +1242,7 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
         w.st = handles.streams[static_cast<size_t>(j)];
         w.done = handles.events[static_cast<size_t>(j)];
         ck(cudaStreamWaitEvent(w.st, R.fork, 0), "fork");
-        ck(ar::launch_rng_init(w.fp, w.base0, w.base1, jb.scene->init_tables, jb.scene->sm_count, w.st), "rng init");
+        ck(ar::launch_rng_init(w.fp, w.base0, w.base1, jb.scene->rng_tables, jb.scene->sm_count, w.st), "rng init");
         ck(ar::launch_render_init(w.ctl, w.total, w.accum, w.npix, w.stats, w.err, jb.scene->sm_count, w.st), "render init");
         ck(cudaEventRecord(w.done, w.st), "event record");
         ck(cudaStreamWaitEvent(st, w.done, 0), "join");
@@ -1303,7 +1297,7 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
         const int gt = kn.trace_bps > 0 ? std::min(jb.scene->grid_trace, jb.scene->sm_count * kn.trace_bps)
                                         : jb.scene->grid_trace;
         const int go = jb.scene->sm_count * (kn.shade_bps > 0 ? kn.shade_bps : 4);
-        ck(ar::launch_iterations(jb.scene->view, w.fp, w.B, w.ctl, w.base0, w.base1, jb.scene->jump_table, w.stats,
+        ck(ar::launch_iterations(jb.scene->view, w.fp, w.B, w.ctl, w.base0, w.base1, jb.scene->rng_tables, w.stats,
                                  w.ovf, w.err, w.accum, nullptr, K, &w.cur, gt, go, w.st, &launches, nullptr),
            "capture iterations");
         ck(ar::launch_tail(jb.scene->view, w.fp, w.B, w.ctl, w.stats, w.ovf, w.err, w.accum, nullptr, w.cur,

@@ -21,6 +21,8 @@ cudaError_t set_intersect_eps_tail(const float* tab9);   // the copy of render_t
 int trace_grid(int sm_count);
 cudaError_t launch_trace_rays(const SceneView& s, const float4* rays, int n, int any, int32_t* obj, float* t,
                               PoolCtl* ctl, uint32_t* ovf, int* err, int grid, cudaStream_t st);
+// The device's copy of xorwow_init_tables() (the first is the frame jump), uploaded when it is not there yet.
+cudaError_t rng_tables(const uint32_t** tables);
 // Per-pixel generator states; tables: xorwow_init_tables() on the device.
 cudaError_t launch_rng_init(const FrameParams& fp, uint4* b0, uint2* b1, const uint32_t* tables, int sm_count, cudaStream_t st);
 cudaError_t launch_rng_tape(const FrameParams& fp, int spp, int per_path, float* out, cudaStream_t st);
