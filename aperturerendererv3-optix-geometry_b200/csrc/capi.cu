@@ -226,10 +226,10 @@ struct ar_scene {
     float bounds[6] = {0, 0, 0, 0, 0, 0};       // box of the BVH root (min xyz, max xyz)
     std::vector<ar::SdfRec> h_sdf;              // data pointers into h_volumes
     std::vector<ar::HostVolume> h_volumes;
-    // render workspace: per-pixel state, counters, traversal overflow
+    // render workspace: per-pixel state, counters, traversal overflow, path state of small renders
     char* ws = nullptr;
     int64_t ws_pix = 0;
-    char* small_paths = nullptr;         // path state of small renders (PathState)
+    char* small_paths = nullptr;
     int64_t small_cap = 0;
     bool counted = false;                // in PathMemory
     uint4* base0 = nullptr;
@@ -259,22 +259,77 @@ struct ar_scene {
         if (ev1) cudaEventDestroy(ev1);
         for (cudaEvent_t e : timer_ext) cudaEventDestroy(e);
         for (cudaEvent_t e : timer_sh) cudaEventDestroy(e);
-        if (small_paths) cudaFree(small_paths);
         if (counted) PathMemory::remove_scene(device);
     }
 };
 
 namespace {
 
-// The path state of one render: up to kSmallPool paths from the scene's own
-// memory (grown as needed), above that PathMemory's block.
+// Frees the workspace; nothing of the scene points into it afterwards, so the
+// scene stays usable when its successor cannot be allocated.
+void drop_workspace(ar_scene* s)
+{
+    if (s->ws) cudaFree(s->ws);
+    s->ws = nullptr;
+    s->ws_pix = 0;
+    s->small_paths = nullptr;
+    s->small_cap = 0;
+    s->rng_valid = false;
+    s->base0 = nullptr;
+    s->base1 = nullptr;
+    s->accum = nullptr;
+    s->fout = nullptr;
+    s->ctl = nullptr;
+    s->stats = nullptr;
+    s->err = nullptr;
+    s->ovf = nullptr;
+}
+
+// Carve the per-pixel buffers, counters and the path state of small renders from
+// one allocation (re-used across calls; grown when a larger image or more paths
+// come).  One, because a new scene's first small render is mostly allocation.
+void ensure_workspace(ar_scene* s, int64_t npix, int64_t paths)
+{
+    if (s->ws && s->ws_pix >= npix && s->small_cap >= paths) return;
+    npix = std::max(npix, s->ws_pix);
+    paths = std::max(paths, s->small_cap);
+    drop_workspace(s);
+    size_t off = 0;
+    auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
+    const size_t N = static_cast<size_t>(npix);
+    const size_t o_b0 = take(16 * N), o_b1 = take(8 * N), o_acc = take(24 * N), o_fout = take(12 * N);
+    const size_t o_cnt = take(sizeof(ar::PoolCtl)), o_stats = take(64), o_err = take(64);
+    const size_t o_ovf = take(static_cast<size_t>(s->grid_trace) * ar::kTraceBlock * ar::kStackOverflow * 4);
+    ar::PathBuffers B{};
+    const size_t o_paths = take(path_layout(B, nullptr, paths));
+    s->ws = dalloc<char>(off, "render workspace");
+    s->ws_pix = npix;
+    char* b = s->ws;
+    s->small_paths = b + o_paths;
+    s->small_cap = paths;
+    s->base0 = reinterpret_cast<uint4*>(b + o_b0);
+    s->base1 = reinterpret_cast<uint2*>(b + o_b1);
+    s->accum = reinterpret_cast<double*>(b + o_acc);
+    s->fout = reinterpret_cast<float*>(b + o_fout);
+    s->ctl = reinterpret_cast<ar::PoolCtl*>(b + o_cnt);
+    s->stats = reinterpret_cast<unsigned long long*>(b + o_stats);
+    s->err = reinterpret_cast<int*>(b + o_err);
+    s->ovf = reinterpret_cast<uint32_t*>(b + o_ovf);
+}
+
+// The path state of one render, with the scene's workspace for it: up to
+// kSmallPool paths (0.12 GB; above the tail kernel's limit, so that renders which
+// run on that kernel alone need no block) from the workspace, above that a block
+// of PathMemory.
 constexpr int64_t kSmallPool = int64_t(1) << 18;
 class PathState {
 public:
     ar::PathBuffers B{};
     // `pool` paths, or fewer when memory is short (down to kSmallPool)
-    PathState(ar_scene* s, int64_t pool, cudaStream_t st) : s_(s), st_(st)
+    PathState(ar_scene* s, int64_t npix, int64_t pool, cudaStream_t st) : s_(s), st_(st)
     {
+        // first: where memory is short the pixels have to fit, the paths may be fewer
+        ensure_workspace(s, npix, pool > kSmallPool ? 0 : pool);
         while (pool > kSmallPool) {
             bytes_ = path_layout(B, nullptr, pool);
             mem_ = PathMemory::take(s->device, bytes_);
@@ -284,13 +339,7 @@ public:
             }
             pool = std::max(kSmallPool, (pool + 1) / 2);
         }
-        if (s->small_cap < pool) {
-            if (s->small_paths) cudaFree(s->small_paths);
-            s->small_paths = nullptr;
-            s->small_cap = 0;
-            s->small_paths = dalloc<char>(path_layout(B, nullptr, pool), "path state");
-            s->small_cap = pool;
-        }
+        ensure_workspace(s, npix, pool);
         path_layout(B, s->small_paths, pool);
     }
     ~PathState()
@@ -307,49 +356,6 @@ private:
     size_t bytes_ = 0;
     cudaStream_t st_;
 };
-
-// Frees the workspace; nothing of the scene points into it afterwards, so the
-// scene stays usable when its successor cannot be allocated.
-void drop_workspace(ar_scene* s)
-{
-    if (s->ws) cudaFree(s->ws);
-    s->ws = nullptr;
-    s->ws_pix = 0;
-    s->rng_valid = false;
-    s->base0 = nullptr;
-    s->base1 = nullptr;
-    s->accum = nullptr;
-    s->fout = nullptr;
-    s->ctl = nullptr;
-    s->stats = nullptr;
-    s->err = nullptr;
-    s->ovf = nullptr;
-}
-
-// Carve the per-pixel buffers and counters from one allocation (re-used across
-// calls; grown when a larger image comes).
-void ensure_workspace(ar_scene* s, int64_t npix)
-{
-    if (s->ws && s->ws_pix >= npix) return;
-    drop_workspace(s);
-    size_t off = 0;
-    auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
-    const size_t N = static_cast<size_t>(npix);
-    const size_t o_b0 = take(16 * N), o_b1 = take(8 * N), o_acc = take(24 * N), o_fout = take(12 * N);
-    const size_t o_cnt = take(sizeof(ar::PoolCtl)), o_stats = take(64), o_err = take(64);
-    const size_t o_ovf = take(static_cast<size_t>(s->grid_trace) * ar::kTraceBlock * ar::kStackOverflow * 4);
-    s->ws = dalloc<char>(off, "render workspace");
-    s->ws_pix = npix;
-    char* b = s->ws;
-    s->base0 = reinterpret_cast<uint4*>(b + o_b0);
-    s->base1 = reinterpret_cast<uint2*>(b + o_b1);
-    s->accum = reinterpret_cast<double*>(b + o_acc);
-    s->fout = reinterpret_cast<float*>(b + o_fout);
-    s->ctl = reinterpret_cast<ar::PoolCtl*>(b + o_cnt);
-    s->stats = reinterpret_cast<unsigned long long*>(b + o_stats);
-    s->err = reinterpret_cast<int*>(b + o_err);
-    s->ovf = reinterpret_cast<uint32_t*>(b + o_ovf);
-}
 
 // intersection::Overlap (intersection.cuh:399-414) at the camera position; the
 // reference scans every object per path, here it is done once per render.
@@ -473,8 +479,7 @@ ar_status run_render(ar_scene* s, const ar_camera* cam, const ar_render_params* 
         fp.guide = *guide;
     }
     if (dn) fp.dn = *dn;
-    ensure_workspace(s, npix);
-    PathState state(s, pool, st);
+    PathState state(s, npix, pool, st);
     const PathBuffers& B = state.B;
     pool = B.capacity;
     fp.pool = static_cast<int32_t>(pool);
@@ -1397,7 +1402,7 @@ ar_status ar_trace_rays(ar_scene* s, const float* rays, size_t n, int32_t any_hi
     AR_GUARD_BEGIN
     DeviceGuard g(s->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    ensure_workspace(s, 1);
+    ensure_workspace(s, 1, 1);
     ck(cudaMemsetAsync(s->err, 0, 64, st), "memset err");
     const float4* drays;
     int32_t* dobj;
