@@ -460,6 +460,17 @@ ar::FrameParams make_frame(const ar_scene* s, const ar_camera* c, const ar_rende
     return fp;
 }
 
+// Renders wait for the device and read counters back, which a stream under
+// capture cannot do.  Refused before anything is enqueued: a small render would
+// otherwise be recorded whole and fail only at its end, with the generator states
+// noted as advanced by kernels that never ran.
+void refuse_capture(cudaStream_t st)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    ck(cudaStreamIsCapturing(st, &c), "render stream");
+    if (c != cudaStreamCaptureStatusNone) throw CudaError(cudaErrorStreamCaptureUnsupported, "render stream");
+}
+
 ar_status run_render(ar_scene* s, const ar_camera* cam, const ar_render_params* p, ar_path_record* rec_dev,
                      cudaStream_t st, ar_render_stats* stats, const ar::NrcFrame* nrc = nullptr,
                      const ar::GuideView* guide = nullptr, const ar::DenoiseView* dn = nullptr)
@@ -467,6 +478,7 @@ ar_status run_render(ar_scene* s, const ar_camera* cam, const ar_render_params* 
     using namespace ar;
     if (p->spectral && !s->spec_tables)
         return fail(AR_ERR_UNSUPPORTED, "spectral rendering needs ar_scene_set_spectral first");
+    refuse_capture(st);
     ar::FrameParams fp = make_frame(s, cam, p);
     const int64_t npix = fp.npix;
     const int64_t total = npix * p->spp;
@@ -1183,6 +1195,7 @@ ar_status render_batch(const ar_job* jobs, int32_t njobs, BatchKnobs kn, ar_batc
     AR_GUARD_BEGIN
     DeviceGuard g(s0->device);
     cudaStream_t user = static_cast<cudaStream_t>(stream);
+    refuse_capture(user);
     // In-flight paths: a shared budget split by each job's share of the work
     // (a job never gets more than it has paths, nor fewer than 2^14).
     int64_t totalAll = 0;
