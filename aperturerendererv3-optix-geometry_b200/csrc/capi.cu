@@ -1415,7 +1415,7 @@ ar_status ar_trace_rays(ar_scene* s, const float* rays, size_t n, int32_t any_hi
     AR_GUARD_BEGIN
     DeviceGuard g(s->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    ensure_workspace(s, 1, 1);
+    ensure_workspace(s, 1, 0);
     ck(cudaMemsetAsync(s->err, 0, 64, st), "memset err");
     const float4* drays;
     int32_t* dobj;
