@@ -1987,10 +1987,11 @@ ar_status ar_batch_autotune(const ar_job* jobs, int32_t njobs, int32_t probe_spp
     const int32_t tbs[3] = {0, 4, 2};   // traversal blocks per SM (0: the kernels' occupancy)
     const int32_t sbs[3] = {4, 2, 1};   // shading / generation / retirement blocks per SM
     ar_batch_stats st;
-    // first use of every workspace (allocations, graph set-up) outside the timing
+    // first use of every workspace (allocations, graph set-up) outside the timing:
+    // the candidates' largest, which the smaller ones then find idle
     BatchKnobs cur;
     cur.iterations = 16;
-    cur.budget = bs[2];
+    cur.budget = bs[3];
     if (ar_status e = render_batch(probe.data(), njobs, cur, &st, stream)) return e;
     ar_batch_tuning best{16, 0, bs[2], 0.0f, 0.0f, 0, 4};
     BatchKnobs bestk = cur;
