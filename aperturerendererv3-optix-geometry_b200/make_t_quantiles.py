@@ -64,6 +64,8 @@ def main() -> None:
     shares = share_threshold(thr)
     least = share_threshold(np.zeros(1, np.float32))[0]
     lines = ["// Generated by make_t_quantiles.py: Student t quantile 0.9975 for nu = 1..1024 (float32).",
+             "// The filter reads the shares alone; the quantiles and the thresholds they derive from",
+             "// are kept for the checks against their published definition.",
              "#pragma once", "", "namespace ar {", "", "constexpr int kTQuantiles = 1024;",
              "static __device__ const float kTQuantile005[kTQuantiles] = {"]
     for k in range(0, len(vals), 6):

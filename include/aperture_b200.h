@@ -244,6 +244,8 @@ ar_status ar_bvh_build_info(const ar_object_desc* objects, size_t count, const a
  *             is ADDED to (resume/extend a render), never cleared
  *   mem_kind  AR_MEM_HOST or AR_MEM_DEVICE for both buffers
  *   stats     optional counters (NULL to skip)
+ * Waits for the device: refused on a stream under capture, as are batches and
+ * cache, guided and denoiser frames.
  * Memory kept between calls: per scene the pixel state of its largest image (60
  * bytes a pixel) and the path state of small renders (up to 2^18 paths, 0.12 GB);
  * per device the path state of larger renders and of batches, in blocks of up to
@@ -644,9 +646,7 @@ ar_status ar_denoise_record(const float* hits, const float* samples, size_t n, a
  * neighbour whose guide weight is not a number (a pixel whose primary ray
  * never hit has a zero normal) contributes nothing.  hdr_in and hdr_out:
  * width*height*3 floats; all pointers on the device; hdr_out must not alias
- * hdr_in.  The call takes 32 bytes per pixel of stream-ordered scratch
- * (cudaMallocAsync / cudaFreeAsync on `stream`) for the tap mask between its
- * two passes. */
+ * hdr_in.  One kernel on `stream`; nothing is allocated. */
 ar_status ar_denoise_bilateral(const float* hdr_in, float* hdr_out, const ar_screen_gbuffer* gbuffer,
                                const ar_screen_stats* stats, int32_t width, int32_t height, void* stream);
 
